@@ -101,6 +101,12 @@ struct pg_ctx {
     cudaEvent_t ev[6] = {};
     std::string err;
     DevBuf cols, bins, dofbuf, par, mi, nlogn, tiles, errw, scratch, counts, edges, mistscr;
+    // sorted-list kernel: frame-major bins, frame lists and segment starts of a
+    // batch of rows, items (of all batches), counter and overflow sums
+    DevBuf smat, slist, sitems, sscr;
+    std::vector<SortedItem> sitems_host;
+    std::vector<int64_t> sitems_cut;  // first item of every row batch, and the end
+    int64_t sitems_key[3] = {-1, -1, -1};
     int nlogn_max = -1;
     DevBuf nfix;          // fixed-point n ln n table of the histogram kernel
     int nfix_max = -1;
@@ -182,12 +188,19 @@ static DofArrays dof_arrays(pg_ctx *ctx, int D) { return dof_at(ctx->dofbuf.p, D
 
 static size_t elem_size(int prec) { return prec ? 8 : 4; }
 
+// Upload groups of host trajectories (run_streamed)
+static int stream_groups() {
+    const char *e = getenv("PG_STREAM_GROUPS");
+    return e ? std::max(1, std::min(pg_ctx::kMaxGroups, atoi(e))) : 1;
+}
+
 // Validation and the geometry of a trajectory (ctx->geo).
-static void set_bin_layout(SysGeom &g, int form);
+static void set_bin_layout(SysGeom &g, int form, bool sorted);
 
 // form: the form the caller asked for (PG_FORM_AUTO/HIST/ONEHOT); it decides
-// the bin-matrix layout the preprocessing writes (set_bin_layout).
-static int setup_geometry(pg_ctx *ctx, const pg_bat_view *tv, const int bins[6], int form) {
+// the bin-matrix layout the preprocessing writes (set_bin_layout). whole: every
+// pair of the system is counted by this call.
+static int setup_geometry(pg_ctx *ctx, const pg_bat_view *tv, const int bins[6], int form, bool whole) {
     if (!tv || !bins) return fail(ctx, PG_ERR_ARG, "null trajectory or bins");
     if (tv->n_dihedrals < 0 || tv->n_frames < 1)
         return fail(ctx, PG_ERR_ARG, "n_dihedrals (%d) < 0 or n_frames (%d) < 1", tv->n_dihedrals, tv->n_frames);
@@ -212,7 +225,7 @@ static int setup_geometry(pg_ctx *ctx, const pg_bat_view *tv, const int bins[6],
     g.F = tv->n_frames;
     g.ldb = bins_ld(g.F);
     for (int k = 0; k < 6; k++) g.bins[k] = bins[k];
-    set_bin_layout(g, form);
+    set_bin_layout(g, form, whole && sorted_layout({g}));
     ctx->resident = false;
     return PG_OK;
 }
@@ -293,8 +306,8 @@ static int queue_ahead(pg_ctx *ctx, cudaStream_t after) {
 }
 
 // preprocessing. Leaves bins, dof arrays and the nlogn table on the device.
-static int run_prep(pg_ctx *ctx, const pg_bat_view *tv, const int bins[6], int form) {
-    int rc0 = setup_geometry(ctx, tv, bins, form);
+static int run_prep(pg_ctx *ctx, const pg_bat_view *tv, const int bins[6], int form, bool whole) {
+    int rc0 = setup_geometry(ctx, tv, bins, form, whole);
     if (rc0) return rc0;
     const SysGeom &g = ctx->geo;
     const int D = g.D;
@@ -411,13 +424,14 @@ static bool use_hist32(const SysGeom &g) { return hist_layout(g) != HIST16; }
 
 // The bin matrices the preprocessing writes for a form: the 16-bit 32-slot
 // layouts stage their row DOFs from the row-code matrix; the streamed layout
-// reads both matrices frame-group interleaved; the one-hot form and the
-// 16-slot kernel read plain DOF rows.
-static void set_bin_layout(SysGeom &g, int form) {
+// reads both matrices frame-group interleaved; the one-hot form, the 16-slot
+// kernel and the sorted-list kernel (whole systems only) read plain DOF rows.
+static void set_bin_layout(SysGeom &g, int form, bool sorted) {
     int chosen = form == PG_FORM_AUTO ? autotune_form(g) : form;
     if (chosen == PG_FORM_ONEHOT && !pairs_onehot_supported(g)) chosen = PG_FORM_HIST;
     const bool hist = chosen != PG_FORM_ONEHOT;
-    const int layout = hist ? hist_layout(g) : HIST16;
+    g.sorted = hist && sorted;
+    const int layout = hist && !g.sorted ? hist_layout(g) : HIST16;
     g.codes = layout_codes(layout, bmax_of(g));
     g.ilv = layout_ilv(layout);
 }
@@ -459,6 +473,108 @@ static int run_hist32(pg_ctx *ctx, const SysGeom &g, const DofArrays &dof, const
     if (explicit_tiles) {
         CK(cudaStreamSynchronize(st));  // the private tile buffer is released on return
     }
+    return PG_OK;
+}
+
+// The same with the 16-slot kernel, over its full tile list.
+static int run_hist16(pg_ctx *ctx, const SysGeom &g, const DofArrays &dof, const PairOut &po) {
+    cudaStream_t st = ctx->stream;
+    int T = 0, fc = 0, nst = 0;
+    if (!pairs_hist_config(bmax_of(g), &T, &fc, &nst)) return fail(ctx, PG_ERR_UNSUPPORTED, "2D bins too large");
+    if (ctx->tiles_D != g.D || ctx->tiles_T != T) {
+        ctx->tiles_host = build_tiles(g.D, T);
+        CK(ctx->tiles.ensure(ctx->tiles_host.size() * sizeof(PairTile)));
+        CK(cudaMemcpyAsync(ctx->tiles.p, ctx->tiles_host.data(), ctx->tiles_host.size() * sizeof(PairTile),
+                           cudaMemcpyHostToDevice, st));
+        CK(cudaStreamSynchronize(st));  // host vector may be rebuilt later
+        ctx->tiles_D = g.D;
+        ctx->tiles_T = T;
+    }
+    const int rc = ensure_fix_table(ctx, g.F);
+    if (rc) return rc;
+    CK(launch_pairs_hist(g, (const uint8_t *)ctx->bins.p, dof, (const unsigned long long *)ctx->nfix.p,
+                         ctx->nfix_scale, (const PairTile *)ctx->tiles.p, (int64_t)ctx->tiles_host.size(), T, po,
+                         (int *)ctx->errw.p, st));
+    ctx->launches++;
+    return PG_OK;
+}
+
+// Every pair of the preprocessed system with the sorted-list kernel. The
+// frame lists take 4 bytes per value, so they are made for batches of rows of
+// at most 16 GB (less where the device has less left). *done is false if not
+// even that fits: the 16-slot kernel reads the same bins.
+static int run_sorted(pg_ctx *ctx, const SysGeom &g, const DofArrays &dof, const PairOut &po, bool *done) {
+    cudaStream_t st = ctx->stream;
+    *done = false;
+    const int bm = bmax_of(g);
+    const int64_t ld = sorted_list_ld(g);
+    const size_t per_row = (size_t)ld * sizeof(uint32_t) + kSegLd * sizeof(int);
+    int rows = (int)std::max<size_t>(1, std::min<size_t>((size_t)g.D, ((size_t)16 << 30) / per_row));
+    cudaError_t e = ctx->smat.ensure(sorted_mat_bytes(g));
+    if (e == cudaSuccess)
+        while ((e = ctx->slist.ensure((size_t)rows * per_row)) == cudaErrorMemoryAllocation && rows > 64) {
+            cudaGetLastError();
+            rows = (rows + 1) / 2;
+        }
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        ctx->smat.release();
+        return PG_OK;
+    }
+    CK(e);
+    const bool big = sorted_ovf_bytes(g) > 0;
+    if (sorted_ovf_bytes(g) + 256 > ctx->sscr.n) {
+        CK(ctx->sscr.ensure(sorted_ovf_bytes(g) + 256));
+        CK(cudaMemsetAsync(ctx->sscr.p, 0, ctx->sscr.n, st));  // launches leave the sums zeroed
+    }
+    int rc = ensure_fix_table(ctx, g.F);
+    if (rc) return rc;
+    SortedArgs a{};
+    SortedSys &d = a.one;
+    d.geo = g;
+    d.dof = dof;
+    d.out = po;
+    d.lnN = log((double)g.F);
+    d.bins = (const uint8_t *)ctx->bins.p;
+    d.mat = (uint8_t *)ctx->smat.p;
+    d.list = (uint32_t *)ctx->slist.p;
+    d.seg = (int *)(d.list + (size_t)rows * ld);
+    d.list_ld = ld;
+    d.pad = sorted_pad(g.D);
+    d.parts = sorted_parts(g, sorted_units(g.D));
+    a.counter = (int *)ctx->sscr.p;
+    a.ovf = (uint32_t *)((char *)ctx->sscr.p + 256);
+    a.nfix = (const unsigned long long *)ctx->nfix.p;
+    a.fix = ctx->nfix_scale;
+    const int64_t key[3] = {g.D, d.parts, rows};
+    if (memcmp(key, ctx->sitems_key, sizeof key) != 0) {
+        ctx->sitems_key[0] = -1;
+        ctx->sitems_host.clear();
+        ctx->sitems_cut.assign(1, 0);
+        for (int r = 0; r < g.D; r += rows) {
+            sorted_items(0, g.D, r, std::min(g.D, r + rows), d.parts, ctx->sitems_host);
+            ctx->sitems_cut.push_back((int64_t)ctx->sitems_host.size());
+        }
+        const size_t nb = ctx->sitems_host.size() * sizeof(SortedItem);
+        CK(ctx->sitems.ensure(nb));
+        CK(cudaMemcpyAsync(ctx->sitems.p, ctx->sitems_host.data(), nb, cudaMemcpyHostToDevice, st));
+        CK(cudaStreamSynchronize(st));  // host vector may be rebuilt later
+        memcpy(ctx->sitems_key, key, sizeof key);
+    }
+    CK(cudaMemsetAsync(po.mi, 0, (size_t)g.D * g.D * sizeof(double), st));
+    CK(launch_sorted_transpose(a, bm, g.F, nullptr, sorted_blocks(g.D), st));
+    ctx->launches++;
+    for (int k = 0; k * (int64_t)rows < g.D; k++) {
+        d.row_first = k * rows;
+        CK(launch_sorted_lists(a, bm, nullptr, d.row_first, std::min(rows, g.D - d.row_first), st));
+        a.items = (const SortedItem *)ctx->sitems.p + ctx->sitems_cut[k];
+        a.n_items = (int)(ctx->sitems_cut[k + 1] - ctx->sitems_cut[k]);
+        CK(launch_pairs_sorted(a, bm, big, st));
+        ctx->launches += 2;
+    }
+    CK(launch_sorted_finish(a, 1, g.D, st));
+    ctx->launches++;
+    *done = true;
     return PG_OK;
 }
 
@@ -511,6 +627,7 @@ static void shard_range(const std::vector<PairTile> &tl, int shard, int n_shards
 // (geometry already set by setup_geometry).
 static int run_streamed(pg_ctx *ctx, const pg_bat_view *tv, pg_par_body *out) {
     const SysGeom &g = ctx->geo;
+    const bool tiled = !g.sorted;  // the sorted-list kernel has no tile list and runs on the context's stream
     const int D = g.D;
     cudaStream_t st = ctx->stream, cs = ctx->copy;
     const size_t es = elem_size(tv->double_prec);
@@ -527,7 +644,7 @@ static int run_streamed(pg_ctx *ctx, const pg_bat_view *tv, pg_par_body *out) {
     CK(ctx->par.ensure((size_t)L.total * sizeof(double)));
     CK(ctx->mi.ensure((size_t)D * D * sizeof(double)));
     const int layout = h32 ? 32 : T;
-    if (ctx->tiles_D != D || ctx->tiles_T != layout) {
+    if (tiled && (ctx->tiles_D != D || ctx->tiles_T != layout)) {
         ctx->tiles_host = h32 ? build_tiles32(D) : build_tiles(D, T);
         CK(ctx->tiles.ensure(ctx->tiles_host.size() * sizeof(PairTile)));
         CK(cudaMemcpyAsync(ctx->tiles.p, ctx->tiles_host.data(), ctx->tiles_host.size() * sizeof(PairTile),
@@ -547,13 +664,11 @@ static int run_streamed(pg_ctx *ctx, const pg_bat_view *tv, pg_par_body *out) {
     // preprocessing waited for SMs the persistent pair kernels held: 16
     // groups took 3.64-3.72 s against 3.58 s for one (copy engine) and 3.45 s
     // with the columns already resident.
-    int K = 1;
-    if (const char *e = getenv("PG_STREAM_GROUPS")) K = std::max(1, std::min(pg_ctx::kMaxGroups, atoi(e)));
-    K = std::min(K, nsb);
+    const int K = tiled ? std::min(stream_groups(), nsb) : 1;
     std::vector<int> G((size_t)K + 1);
     std::vector<int64_t> cut((size_t)K + 1);
     for (int k = 0; k <= K; k++) G[k] = std::min(D, (int)((int64_t)k * nsb / K) * sbw);
-    {
+    if (tiled) {
         const std::vector<PairTile> &tl = ctx->tiles_host;
         int64_t i = 0;
         for (int k = 0; k <= K; k++) {
@@ -561,10 +676,10 @@ static int run_streamed(pg_ctx *ctx, const pg_bat_view *tv, pg_par_body *out) {
             cut[k] = k == K ? (int64_t)tl.size() : i;
         }
     }
-    const size_t sb32 = h32 ? pairs_hist32_scratch_bytes(bmax_of(g), pairs_hist32_grid((int64_t)ctx->tiles_host.size()))
+    const size_t sb32 = h32 && tiled ? pairs_hist32_scratch_bytes(bmax_of(g), pairs_hist32_grid((int64_t)ctx->tiles_host.size()))
                             : 0;
     // one scratch area (tile counter, overflow counts) per pair stream
-    if (h32) CK(ctx->scratch.ensure(2 * sb32));
+    if (h32 && tiled) CK(ctx->scratch.ensure(2 * sb32));
 
     CK(cudaEventRecord(ctx->ev[0], st));
     CK(cudaStreamWaitEvent(cs, ctx->ev[0], 0));  // earlier kernels reading the columns are done
@@ -624,6 +739,13 @@ static int run_streamed(pg_ctx *ctx, const pg_bat_view *tv, pg_par_body *out) {
         CK(launch_prep(g, colp, F, tv->double_prec, dof, (uint8_t *)ctx->bins.p, (int *)ctx->errw.p, st, G[k],
                        G[k + 1] - G[k]));
         ctx->launches++;
+        if (!tiled) {
+            bool done = false;
+            rc = run_sorted(ctx, g, dof, po, &done);
+            if (!rc && !done) rc = run_hist16(ctx, g, dof, po);
+            if (rc) return rc;
+            break;
+        }
         // group k's pair tiles need the bins of groups 0..k: every prep so far
         CK(cudaEventRecord(ctx->pev[k], st));
         const int64_t n = cut[k + 1] - cut[k];
@@ -701,7 +823,7 @@ PG_API void pg_destroy(pg_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->pf_pending) cudaEventSynchronize(ctx->pf_done);
     for (DevBuf *b : {&ctx->cols, &ctx->cols_pf, &ctx->bins, &ctx->dofbuf, &ctx->par, &ctx->mi, &ctx->nlogn, &ctx->nfix,
-                      &ctx->tiles, &ctx->errw, &ctx->scratch, &ctx->counts, &ctx->edges, &ctx->mistscr,
+                      &ctx->tiles, &ctx->errw, &ctx->scratch, &ctx->smat, &ctx->slist, &ctx->sitems, &ctx->sscr, &ctx->counts, &ctx->edges, &ctx->mistscr,
                       &ctx->bc_out, &ctx->bc_stage, &ctx->bc_soa, &ctx->bc_tmp, &ctx->bc_tab, &ctx->mie_body,
                       &ctx->mie_slots, &ctx->mie_lens, &ctx->mie_rows, &ctx->mie_text, &ctx->mie_fb})
         b->release();
@@ -969,12 +1091,12 @@ PG_API int pg_entropy(pg_ctx *ctx, const pg_bat_view *traj, const int bins[6], i
     cudaGetLastError();  // an error left by an earlier failed call of this thread is not this call's
     if (form < PG_FORM_AUTO || form > PG_FORM_ONEHOT) return fail(ctx, PG_ERR_ARG, "unknown form %d", form);
     if (traj && !traj->on_device && form != PG_FORM_ONEHOT) {
-        int rc0 = setup_geometry(ctx, traj, bins, form);
+        int rc0 = setup_geometry(ctx, traj, bins, form, stream_groups() == 1);
         if (rc0) return rc0;
         const int f = form == PG_FORM_AUTO ? autotune_form(ctx->geo) : form;
         if (f != PG_FORM_ONEHOT || !pairs_onehot_supported(ctx->geo)) return run_streamed(ctx, traj, out);
     }
-    int rc = run_prep(ctx, traj, bins, form);
+    int rc = run_prep(ctx, traj, bins, form, true);
     if (rc) return rc;
     const SysGeom &g = ctx->geo;
     cudaStream_t st = ctx->stream;
@@ -999,28 +1121,17 @@ PG_API int pg_entropy(pg_ctx *ctx, const pg_bat_view *traj, const int bins[6], i
     po.L = L;
     po.counts = nullptr;
     po.counts_bmax = 0;
-    if (chosen == PG_FORM_HIST && use_hist32(g)) {
-        int rc2 = run_hist32(ctx, g, dof, po, nullptr, 0);
-        if (rc2) return rc2;
-    } else if (chosen == PG_FORM_HIST) {
-        int T = 0, fc = 0, nst = 0;
-        if (!pairs_hist_config(bmax_of(g), &T, &fc, &nst)) return fail(ctx, PG_ERR_UNSUPPORTED, "2D bins too large");
-        if (ctx->tiles_D != g.D || ctx->tiles_T != T) {
-            ctx->tiles_host = build_tiles(g.D, T);
-            CK(ctx->tiles.ensure(ctx->tiles_host.size() * sizeof(PairTile)));
-            CK(cudaMemcpyAsync(ctx->tiles.p, ctx->tiles_host.data(), ctx->tiles_host.size() * sizeof(PairTile),
-                               cudaMemcpyHostToDevice, st));
-            CK(cudaStreamSynchronize(st));  // host vector may be rebuilt later
-            ctx->tiles_D = g.D;
-            ctx->tiles_T = T;
+    if (chosen == PG_FORM_HIST) {
+        bool done = false;
+        if (g.sorted) {
+            const int rcs = run_sorted(ctx, g, dof, po, &done);
+            if (rcs) return rcs;
         }
-        int rc3 = ensure_fix_table(ctx, g.F);
-        if (rc3) return rc3;
-        CK(launch_pairs_hist(g, (const uint8_t *)ctx->bins.p, dof, (const unsigned long long *)ctx->nfix.p,
-                             ctx->nfix_scale,
-                             (const PairTile *)ctx->tiles.p, (int64_t)ctx->tiles_host.size(), T, po,
-                             (int *)ctx->errw.p, st));
-        ctx->launches++;
+        if (!done) {
+            const int rch = !g.sorted && use_hist32(g) ? run_hist32(ctx, g, dof, po, nullptr, 0)
+                                                       : run_hist16(ctx, g, dof, po);
+            if (rch) return rch;
+        }
     } else {
         const size_t sb = pairs_onehot_scratch_bytes(g);
         CK(ctx->scratch.ensure(sb));
@@ -1106,7 +1217,7 @@ PG_API int pg_entropy_shard(pg_ctx *ctx, const pg_bat_view *traj, const int bins
     if (n_shards < 1 || shard < 0 || shard >= n_shards) return fail(ctx, PG_ERR_ARG, "shard %d of %d", shard, n_shards);
     if (form == PG_FORM_ONEHOT) return fail(ctx, PG_ERR_UNSUPPORTED, "shards use the histogram form");
     if (form != PG_FORM_AUTO && form != PG_FORM_HIST) return fail(ctx, PG_ERR_ARG, "unknown form %d", form);
-    int rc = run_prep(ctx, traj, bins, PG_FORM_HIST);  // every shard bins all D columns (O(D F))
+    int rc = run_prep(ctx, traj, bins, PG_FORM_HIST, false);  // every shard bins all D columns (O(D F))
     if (rc) return rc;
     const SysGeom &g = ctx->geo;
     cudaStream_t st = ctx->stream;
@@ -1165,7 +1276,7 @@ PG_API int pg_pair_counts(pg_ctx *ctx, const pg_bat_view *traj, const int bins[6
     cudaGetLastError();  // an error left by an earlier failed call of this thread is not this call's
     if (n_pairs < 0 || (n_pairs > 0 && (!g1 || !g2 || !counts))) return fail(ctx, PG_ERR_ARG, "bad pair list");
     if (form == PG_FORM_ONEHOT) return fail(ctx, PG_ERR_UNSUPPORTED, "count export uses the histogram form");
-    int rc = run_prep(ctx, traj, bins, PG_FORM_HIST);
+    int rc = run_prep(ctx, traj, bins, PG_FORM_HIST, false);
     if (rc) return rc;
     const SysGeom &g = ctx->geo;
     std::vector<PairTile> t((size_t)n_pairs);
@@ -1466,7 +1577,7 @@ struct BatchLayout {
     SysGeom g;
     int prec = 0;
     int64_t ld = 0;
-    size_t cols = 0, bins = 0, dof = 0, par = 0, mi = 0, mist = 0, edges = 0;
+    size_t cols = 0, bins = 0, dof = 0, par = 0, mi = 0, mist = 0, edges = 0, mat = 0, list = 0, seg = 0;
     bool own_cols = false;
 };
 
@@ -1503,7 +1614,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
     // The form of the batch: one form for every system, in one pair launch.
     // Automatically the one-hot form where the autotuner picks it for every
     // system (the batched one-hot launch runs every system's tiles together).
-    bool onehot = form == PG_FORM_ONEHOT;
+    bool onehot = form == PG_FORM_ONEHOT, srt = false;
     {
         bool all_supported = true;
         std::vector<SysGeom> geos((size_t)n_sys);
@@ -1524,49 +1635,86 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
         if (form == PG_FORM_ONEHOT && !all_supported)
             return fail(ctx, PG_ERR_UNSUPPORTED, "one-hot tensor-core form unsupported for a system of the batch");
         if (form == PG_FORM_AUTO) onehot = autotune_batch_form(geos) == PG_FORM_ONEHOT;
+        srt = !onehot && sorted_layout(geos);
     }
 
-    // ---- layout of every system inside one arena
+    // ---- layout of every system inside one arena; the MI matrices of all
+    // systems are one range of it
     std::vector<BatchLayout> sys((size_t)n_sys);
-    size_t off = 0;
+    size_t off = 0, mi_begin = 0, mi_end = 0;
     int maxF = 1, maxD = 1;
-    for (int s = 0; s < n_sys; s++) {
-        const pg_bat_view &v = trajs[s];
-        int rc = validate_view(ctx, &v, s);
-        if (rc) return rc;
-        BatchLayout &L = sys[s];
-        SysGeom &g = L.g;
-        g.n_dih = v.n_dihedrals;
-        g.nb = g.n_dih + 2;
-        g.na = g.n_dih + 1;
-        g.nd = g.n_dih;
-        g.D = g.nb + g.na + g.nd;
-        g.F = v.n_frames;
-        g.ldb = bins_ld(g.F);
-        for (int k = 0; k < 6; k++) g.bins[k] = bins[k];
-        set_bin_layout(g, onehot ? PG_FORM_ONEHOT : PG_FORM_HIST);
-        L.prec = v.double_prec;
-        L.own_cols = !v.on_device;
-        L.ld = v.on_device ? v.ld : v.n_frames;
-        if (L.own_cols) {
-            L.cols = off;
-            off = al256(off + (size_t)g.D * g.F * elem_size(v.double_prec));
+    auto lay_out = [&](bool sorted) {
+        off = 0;
+        size_t lists = 0;
+        for (int s = 0; s < n_sys; s++) {
+            const pg_bat_view &v = trajs[s];
+            BatchLayout &L = sys[s];
+            L = BatchLayout{};
+            SysGeom &g = L.g;
+            g.n_dih = v.n_dihedrals;
+            g.nb = g.n_dih + 2;
+            g.na = g.n_dih + 1;
+            g.nd = g.n_dih;
+            g.D = g.nb + g.na + g.nd;
+            g.F = v.n_frames;
+            g.ldb = bins_ld(g.F);
+            for (int k = 0; k < 6; k++) g.bins[k] = bins[k];
+            set_bin_layout(g, onehot ? PG_FORM_ONEHOT : PG_FORM_HIST, sorted);
+            L.prec = v.double_prec;
+            L.own_cols = !v.on_device;
+            L.ld = v.on_device ? v.ld : v.n_frames;
+            if (L.own_cols) {
+                L.cols = off;
+                off = al256(off + (size_t)g.D * g.F * elem_size(v.double_prec));
+            }
+            L.bins = off;
+            off = al256(off + bins_bytes(g));
+            L.dof = off;
+            off = al256(off + dof_bytes(g.D));
+            L.par = off;
+            off = al256(off + (size_t)par_layout(g.n_dih).total * sizeof(double));
+            L.mist = off;
+            off = al256(off + mist_scratch_bytes(g.D));
+            L.edges = off;
+            off = al256(off + (size_t)g.D * (sizeof(double) + 2 * sizeof(int)));
+            if (g.sorted) {
+                L.mat = off;
+                off = al256(off + sorted_mat_bytes(g));
+                L.list = off;
+                off = al256(off + (size_t)g.D * sorted_list_ld(g) * sizeof(uint32_t));
+                L.seg = off;
+                off = al256(off + (size_t)g.D * kSegLd * sizeof(int));
+                lists += (size_t)g.D * sorted_list_ld(g) * sizeof(uint32_t);
+            }
+            maxF = std::max(maxF, g.F);
+            maxD = std::max(maxD, g.D);
         }
-        L.bins = off;
-        off = al256(off + bins_bytes(g));
-        L.dof = off;
-        off = al256(off + dof_bytes(g.D));
-        L.par = off;
-        off = al256(off + (size_t)par_layout(g.n_dih).total * sizeof(double));
-        L.mi = off;
-        off = al256(off + (size_t)g.D * g.D * sizeof(double));
-        L.mist = off;
-        off = al256(off + mist_scratch_bytes(g.D));
-        L.edges = off;
-        off = al256(off + (size_t)g.D * (sizeof(double) + 2 * sizeof(int)));
-        maxF = std::max(maxF, g.F);
-        maxD = std::max(maxD, g.D);
+        mi_begin = off;
+        for (BatchLayout &L : sys) {
+            L.mi = off;
+            off = al256(off + (size_t)L.g.D * L.g.D * sizeof(double));
+        }
+        mi_end = off;
+        return lists;
+    };
+    for (int s = 0; s < n_sys; s++) {
+        const int rc = validate_view(ctx, &trajs[s], s);
+        if (rc) return rc;
     }
+    // The sorted-list kernel's frame lists of all systems are held at once
+    // here: beyond 64 GB of them (or of what the device has) the tiled kernels
+    // run instead.
+    srt = srt && lay_out(true) <= ((size_t)64 << 30);
+    if (srt) {
+        const cudaError_t e = ctx->batch.ensure(off);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            srt = false;
+        } else {
+            CK(e);
+        }
+    }
+    if (!srt) lay_out(false);
     if (prep_smem_bytes(sys[0].g) > 200 * 1024) return fail(ctx, PG_ERR_UNSUPPORTED, "1D bin counts too large");
     CK(ctx->batch.ensure(off));
     CK(ctx->errw.ensure(ERR_WORDS * sizeof(int)));
@@ -1576,7 +1724,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
     }
     char *arena = (char *)ctx->batch.p;
     const int bmax = bmax_of(sys[0].g);
-    const bool h32 = use_hist32(sys[0].g);
+    const bool h32 = use_hist32(sys[0].g) && !srt;
     int T = 0, fc = 0, nst = 0;
     if (!pairs_hist_config(bmax, &T, &fc, &nst)) return fail(ctx, PG_ERR_UNSUPPORTED, "2D bins too large");
 
@@ -1611,8 +1759,44 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
     std::vector<int> order((size_t)n_sys);
     for (int s = 0; s < n_sys; s++) order[s] = s;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return sys[a].g.F > sys[b].g.F; });
+    // sorted-list kernel: descriptors, items (of the longest trajectories
+    // first too), and the (system, row) and (system, block) of every CTA of its
+    // preparation
+    std::vector<SortedSys> sos;
+    std::vector<SortedItem> items;
+    std::vector<int2> rmap, bmap;
+    size_t so_ovf = 0;
+    if (srt) {
+        sos.resize((size_t)n_sys);
+        int64_t units = 0;
+        for (int s = 0; s < n_sys; s++) units += sorted_units(sys[s].g.D);
+        for (int s : order) {
+            const BatchLayout &L = sys[s];
+            SortedSys &q = sos[s];
+            q.geo = L.g;
+            q.dof = sd[s].dof;
+            q.out = sd[s].out;
+            q.lnN = sd[s].lnN;
+            q.bins = sd[s].bins;
+            q.mat = (uint8_t *)(arena + L.mat);
+            q.list = (uint32_t *)(arena + L.list);
+            q.seg = (int *)(arena + L.seg);
+            q.list_ld = sorted_list_ld(L.g);
+            q.row_first = 0;
+            q.pad = sorted_pad(L.g.D);
+            q.parts = sorted_parts(L.g, units);
+            sorted_items(s, L.g.D, 0, L.g.D, q.parts, items);
+            for (int r = 0; r < L.g.D; r++) rmap.push_back(make_int2(s, r));
+            for (int b = 0; b < sorted_blocks(L.g.D); b++) bmap.push_back(make_int2(s, b));
+            so_ovf = std::max(so_ovf, sorted_ovf_bytes(L.g));
+        }
+        if (so_ovf + 256 > ctx->sscr.n) {
+            CK(ctx->sscr.ensure(so_ovf + 256));
+            CK(cudaMemsetAsync(ctx->sscr.p, 0, ctx->sscr.n, st));
+        }
+    }
     for (int s : order) {
-        if (onehot) break;  // the one-hot launch builds its own tile list
+        if (onehot || srt) break;  // these launches have their own work lists
         std::vector<PairTile> t = h32 ? build_tiles32(sys[s].g.D) : build_tiles(sys[s].g.D, T);
         tiles.insert(tiles.end(), t.begin(), t.end());
         tsys.insert(tsys.end(), t.size(), s);
@@ -1651,7 +1835,10 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
                  mo_pd = mo_ts + al256(sizeof(int) * std::max<size_t>(tsys.size(), 1)),
                  mo_m0 = mo_pd + al256(sizeof(PrepDesc) * n_sys),
                  mo_m1 = mo_m0 + al256(sizeof(int2) * std::max<size_t>(pmap[0].size(), 1)),
-                 mo_end = mo_m1 + al256(sizeof(int2) * std::max<size_t>(pmap[1].size(), 1));
+                 mo_so = mo_m1 + al256(sizeof(int2) * std::max<size_t>(pmap[1].size(), 1)),
+                 mo_si = mo_so + al256(sizeof(SortedSys) * sos.size()),
+                 mo_rm = mo_si + al256(sizeof(SortedItem) * items.size()),
+                 mo_bm = mo_rm + al256(sizeof(int2) * rmap.size()), mo_end = mo_bm + al256(sizeof(int2) * bmap.size());
     CK(ctx->batchmeta.ensure(mo_end));
     char *meta = (char *)ctx->batchmeta.p;
 
@@ -1669,6 +1856,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
     key.push_back(sys[0].g.codes);
     key.push_back(sys[0].g.ilv);
     key.push_back(onehot ? (int64_t)(uintptr_t)ctx->ohbatch.p : -1);
+    key.push_back(srt ? (int64_t)(uintptr_t)ctx->sscr.p : -1);
     for (int k = 0; k < 6; k++) key.push_back(bins[k]);
     for (int s = 0; s < n_sys; s++) {
         const pg_bat_view &v = trajs[s];
@@ -1691,6 +1879,12 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
             if (!pmap[q].empty())
                 CK(cudaMemcpyAsync(meta + (q ? mo_m1 : mo_m0), pmap[q].data(), sizeof(int2) * pmap[q].size(),
                                    cudaMemcpyHostToDevice, st));
+        if (srt) {
+            CK(cudaMemcpyAsync(meta + mo_so, sos.data(), sizeof(SortedSys) * sos.size(), cudaMemcpyHostToDevice, st));
+            CK(cudaMemcpyAsync(meta + mo_si, items.data(), sizeof(SortedItem) * items.size(), cudaMemcpyHostToDevice, st));
+            CK(cudaMemcpyAsync(meta + mo_rm, rmap.data(), sizeof(int2) * rmap.size(), cudaMemcpyHostToDevice, st));
+            CK(cudaMemcpyAsync(meta + mo_bm, bmap.data(), sizeof(int2) * bmap.size(), cudaMemcpyHostToDevice, st));
+        }
         CK(cudaStreamSynchronize(st));  // host vectors go out of scope
         if (onehot) {
             // descriptors, row tables and n ln n tables of the one-hot launch
@@ -1742,7 +1936,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
         for (int q = 0; q < 2 && e == cudaSuccess; q++)
             e = launch_prep_batch(sys[0].g, (const PrepDesc *)(meta + mo_pd), (const int2 *)(meta + (q ? mo_m1 : mo_m0)),
                                   (int)pmap[q].size(), q, (int *)ctx->errw.p, st);
-        for (int s = 0; s < n_sys && e == cudaSuccess; s++) {
+        for (int s = 0; s < n_sys && e == cudaSuccess && !srt; s++) {
             const BatchLayout &L = sys[s];
             e = cudaMemcpyAsync(arena + L.par, dofs_at(L).s1, (size_t)L.g.D * sizeof(double), cudaMemcpyDeviceToDevice,
                                 st);
@@ -1750,7 +1944,23 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
         int oh_launches = 0;
         if (e == cudaSuccess && onehot)
             e = launch_pairs_onehot_batch(gs, ctx->ohbatch.p, (int *)ctx->errw.p, st, &oh_launches);
-        else if (e == cudaSuccess)
+        else if (e == cudaSuccess && srt) {
+            SortedArgs a{};
+            a.many = (const SortedSys *)(meta + mo_so);
+            a.items = (const SortedItem *)(meta + mo_si);
+            a.n_items = (int)items.size();
+            a.counter = (int *)ctx->sscr.p;
+            a.ovf = (uint32_t *)((char *)ctx->sscr.p + 256);
+            a.nfix = (const unsigned long long *)ctx->nfix.p;
+            a.fix = ctx->nfix_scale;
+            e = cudaMemsetAsync(arena + mi_begin, 0, mi_end - mi_begin, st);
+            if (e == cudaSuccess)
+                e = launch_sorted_transpose(a, bmax, maxF, (const int2 *)(meta + mo_bm), (int)bmap.size(), st);
+            if (e == cudaSuccess)
+                e = launch_sorted_lists(a, bmax, (const int2 *)(meta + mo_rm), 0, (int)rmap.size(), st);
+            if (e == cudaSuccess) e = launch_pairs_sorted(a, bmax, so_ovf > 0, st);
+            if (e == cudaSuccess) e = launch_sorted_finish(a, n_sys, maxD, st);
+        } else if (e == cudaSuccess)
             e = h32 ? launch_pairs_hist32_batch(bmax, sys[0].g.codes != 0, sys[0].g.ilv != 0,
                                                 (const SysDesc *)(meta + mo_sd),
                                                 (const PairTile *)(meta + mo_t),
@@ -1774,7 +1984,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
     }
     CK(cudaGraphLaunch(ctx->graph, st));
     // preps, pair kernel (+ the one-hot finalize), MIST
-    ctx->launches += (pmap[0].empty() ? 0 : 1) + (pmap[1].empty() ? 0 : 1) + (onehot ? 3 : 2);
+    ctx->launches += (pmap[0].empty() ? 0 : 1) + (pmap[1].empty() ? 0 : 1) + (onehot ? 3 : (srt ? 5 : 2));
     CK(cudaEventRecord(ctx->ev[2], st));
     int rc = check_err_words(ctx);
     float ms[2];

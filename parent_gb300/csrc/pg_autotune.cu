@@ -260,12 +260,14 @@ SysGeom as_hist(const SysGeom &g, int layout) {
     SysGeom h = g;
     h.codes = layout_codes(layout, bmax_of(g));
     h.ilv = layout_ilv(layout);
+    h.sorted = 0;
     return h;
 }
 SysGeom as_onehot(const SysGeom &g) {
     SysGeom h = g;
     h.codes = 0;
     h.ilv = 0;
+    h.sorted = 0;
     return h;
 }
 
@@ -295,6 +297,32 @@ int hist_layout(const SysGeom &g) {
     if (e && atoi(e) == 32) return pairs_hist32_supported(bm) ? HIST32_RING : HIST16;
     if (st && atoi(st) == 0) return pairs_hist32_wide(bm) ? HIST32_RING : HIST16;
     return pairs_hist32_supported(bm) ? HIST32_STREAM : HIST16;
+}
+
+// The sorted-list kernel, from pair-phase times against the kernel that
+// hist_layout picks (same system, one call after the other). It counts whole
+// blocks of 128 columns, of which a small system leaves many empty; the line
+// is drawn on the counted slots per pair (2,994 DOFs: 1.04, 894: 1.14, 603:
+// 1.21, 444: 1.29, 294: 1.57, 174: 1.85). 36-50 bins: 2,994 DOFs x 100k frames
+// 90.5 -> 73.8 ms at 50 bins, 894 DOFs 8.2 -> 7.9, 603 DOFs 3.82 -> 4.00.
+// Above 50 bins the other kernel holds 4 pairs per CTA (to 100), then 1: 1,194
+// DOFs x 60k x 90 bins 24.1 -> 10.5 ms; 603 DOFs x 20k x 51 bins 1.37 -> 1.11,
+// 444 DOFs x 5k 0.36 -> 0.38; 294 DOFs x 5k x 64 bins 0.39 -> 0.29, 174 DOFs
+// x 20k 0.24 -> 0.29; 294 DOFs x 5k x 160 bins 1.60 -> 1.21, 174 DOFs 0.57 ->
+// 0.74. A batch counts as one system of all its slots and pairs.
+// PG_HIST_SORTED=0|1 forces it off or on; PG_HIST_SLOTS and PG_HIST_STREAM
+// choose among the other kernels.
+bool sorted_layout(const std::vector<SysGeom> &gs) {
+    if (const char *e = getenv("PG_HIST_SORTED")) return atoi(e) != 0;
+    if (getenv("PG_HIST_SLOTS") || getenv("PG_HIST_STREAM")) return false;
+    double slots = 0.0, pairs = 0.0;
+    int bm = 0;
+    for (const SysGeom &g : gs) {
+        bm = std::max(bm, bmax_of(g));
+        slots += (double)sorted_units(g.D) * 128.0 * g.F;
+        pairs += 0.5 * g.D * (g.D - 1.0) * g.F;
+    }
+    return bm > 35 && slots < pairs * (bm <= 50 ? 1.18 : (bm <= 57 ? 1.25 : 1.7));
 }
 
 int layout_codes(int layout, int bmax) { return layout != HIST16 && !pairs_hist32_wide(bmax) ? 1 : 0; }

@@ -32,6 +32,7 @@ struct SysGeom {
                                // each 2D bin b as the row code (b >> 1) | (b & 1) << 7
     int ilv;                   // 1: both matrices are frame-group interleaved (ilv_index)
                                // instead of DOF rows ldb bytes apart
+    int sorted;                // 1: plain DOF rows, counted by the sorted-list kernel
 };
 
 // Frame-group interleaved bin layout (SysGeom::ilv), read by the streamed
@@ -249,6 +250,56 @@ cudaError_t launch_pairs_hist32_batch(int bmax, bool codes, bool ilv, const SysD
                                       const int *tile_sys, int64_t n_tiles, const unsigned long long *nfix,
                                       double fix, int *err, void *scratch, size_t scratch_bytes, cudaStream_t st);
 
+// Sorted-list histogram pair kernel (pg_pairs_sorted.cu): the frames of every
+// row DOF listed by its 2D bin, the bins of all columns transposed to
+// frame-major rows of 128-column blocks. One call is: launch_sorted_transpose
+// (after the preprocessing), then per batch of rows launch_sorted_lists and
+// launch_pairs_sorted (which adds to the zeroed MI matrix's storage), then
+// launch_sorted_finish (S2D into the body, MI in place of the sums).
+constexpr int kSegLd = 220;  // ints per row of segment starts (at most 218 bins, and the end)
+struct SortedItem {          // segments of share `part` of row x column block
+    int sys, row, blk, part;
+};
+struct SortedSys {
+    SysGeom geo;
+    DofArrays dof;
+    PairOut out;
+    double lnN;
+    const uint8_t *bins;  // DOF rows
+    uint8_t *mat;         // sorted_mat_bytes
+    uint32_t *list;       // rows from row_first, list_ld entries apart
+    int *seg;             // their segment starts, kSegLd apart
+    int64_t list_ld;
+    int row_first;
+    int pad;              // sorted_pad(D)
+    int parts;            // items per (row, block)
+};
+struct SortedArgs {
+    SortedSys one;         // single system (many == nullptr)
+    const SortedSys *many;
+    const SortedItem *items;
+    int n_items;
+    int *counter;          // next item
+    const unsigned long long *nfix;
+    double fix;
+    uint32_t *ovf;         // sorted_ovf_bytes, zeroed; each launch leaves it zeroed
+    int rows, teams, dummy;  // set by the launchers
+};
+int64_t sorted_list_ld(const SysGeom &g);
+int sorted_blocks(int D);
+size_t sorted_mat_bytes(const SysGeom &g);
+int sorted_pad(int D);
+size_t sorted_ovf_bytes(const SysGeom &g);
+int64_t sorted_units(int D);
+int sorted_parts(const SysGeom &g, int64_t units);
+void sorted_items(int s, int D, int row0, int row1, int parts, std::vector<SortedItem> &out);
+cudaError_t launch_sorted_transpose(const SortedArgs &a, int bmax, int max_F, const int2 *map, int n_blocks,
+                                    cudaStream_t st);
+cudaError_t launch_sorted_lists(const SortedArgs &a, int bmax, const int2 *map, int row0, int n_rows, cudaStream_t st);
+// big: a segment can be longer than the 16-bit counters hold (a.ovf is needed)
+cudaError_t launch_pairs_sorted(const SortedArgs &a, int bmax, bool big, cudaStream_t st);
+cudaError_t launch_sorted_finish(const SortedArgs &a, int n_sys, int max_D, cudaStream_t st);
+
 // Cartesian -> BAT conversion (pg_batconv.cu): coordinates of a chunk of
 // frames to one row per (atom, xyz) scaled by 10; bonds/angles/raw dihedrals;
 // phase angles and the [0, 2 pi) shift. Columns ld elements apart, frames f0..
@@ -353,6 +404,10 @@ int64_t pairs_onehot_tiles(const SysGeom &g);
 // straight from the frame-group interleaved bin matrix).
 enum { HIST16 = 0, HIST32_RING = 1, HIST32_STREAM = 2 };
 int hist_layout(const SysGeom &g);
+// Whether a whole-system call (one geometry) or a batch counts its pairs with
+// the sorted-list kernel instead of hist_layout's (shards and count exports
+// keep hist_layout's tiles).
+bool sorted_layout(const std::vector<SysGeom> &gs);
 // SysGeom::codes / SysGeom::ilv of a histogram layout at a bin count
 int layout_codes(int layout, int bmax);
 int layout_ilv(int layout);

@@ -1,0 +1,89 @@
+"""The sorted-list histogram kernel (pg_pairs_sorted.cu) against the tiled
+histogram kernels and the oracle.
+
+Every pair's counts enter exact integer sums, and every kernel finishes with
+the same expressions, so the bodies must agree bit for bit; the oracle's 2D
+entropies are within 1e-9 nats (the bound of the other kernels' tests). Sizes
+are the edges of its tiles: one block of 128 columns less, exact and more, rows
+of 4 frames and batches of 32, counts past a 16-bit half, one frame, and the
+smallest and largest bin counts."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import oracle
+import parent_gb300 as pg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def eng():
+    e = pg.Engine(0)
+    yield e
+    e.close()
+
+
+def _both(eng, monkeypatch, traj, bins):
+    out = []
+    for on in ("1", "0"):
+        monkeypatch.setenv("PG_HIST_SORTED", on)
+        body = eng.entropy(traj, bins, "hist")
+        edges, totals = eng.mist(traj.n_dih if isinstance(traj, pg.Trajectory) else traj.n_dihedrals)
+        out.append((body.flat(), edges, totals))
+    return out
+
+
+# atoms, frames, 2D bins (b, a, d), double precision
+SHAPES = [
+    (3, 5, (50, 50, 50), 0),        # no dihedral: 3 DOFs
+    (5, 1, (40, 40, 40), 1),        # one frame
+    (44, 31, (50, 36, 40), 0),      # 126 DOFs: a block less 2; less than a batch of frames
+    (45, 32, (51, 51, 51), 1),      # 129 DOFs: one column past a block
+    (88, 997, (58, 57, 60), 0),     # 258 DOFs; two and four warps per table
+    (30, 4097, (119, 120, 121), 0), # four and eight warps per table
+    (12, 2049, (218, 218, 218), 1), # the largest table
+    (40, 3000, (1, 2, 3), 0),       # the smallest tables
+    (24, 20001, (50, 50, 50), 0),   # several items per row and block
+]
+
+
+@pytest.mark.parametrize("atoms,frames,b2,prec", SHAPES)
+def test_sorted_equals_tiled_and_oracle(eng, monkeypatch, atoms, frames, b2, prec):
+    bins = (20, 30, 40) + b2
+    t = pg.synth_host(atoms, frames, double_prec=prec, seed=atoms + frames, frac_bimodal_dih=0.3)
+    (a, ea, ta), (b, eb, tb) = _both(eng, monkeypatch, t, bins)
+    assert np.array_equal(a, b)
+    assert np.array_equal(ea, eb) and np.array_equal(ta, tb)
+    r = oracle.parent(t.bonds, t.angles, t.dihedrals, bins)
+    ref = np.concatenate([r[k] for k in oracle.BLOCKS])
+    assert np.max(np.abs(a - ref)) <= 1e-9
+
+
+@pytest.mark.parametrize("frames", [64512, 64513, 140000])
+def test_sorted_counts_above_16_bits(eng, monkeypatch, frames):
+    """Columns with one value in most frames: segments and counts around and
+    past what a 16-bit half holds (pieces of 64,512 frames)."""
+    t = pg.synth_host(9, frames, double_prec=0, seed=5)
+    for k, c in enumerate((t.bonds, t.angles, t.dihedrals)):
+        c[:, : frames - 7 - k] = c[:, :1]
+    (a, ea, _), (b, eb, _) = _both(eng, monkeypatch, t, (50,) * 6)
+    assert np.array_equal(a, b) and np.array_equal(ea, eb)
+
+
+def test_sorted_batch_equals_single_calls(eng, monkeypatch):
+    """One launch over systems of several sizes, replayed, against a call per
+    system (the batch's items are split differently)."""
+    monkeypatch.setenv("PG_HIST_SORTED", "1")
+    bins = (50, 50, 50, 50, 44, 39)
+    trajs = [pg.synth_host(a, f, double_prec=p, seed=k) for k, (a, f, p) in
+             enumerate([(50, 5000, 0), (4, 64600, 1), (90, 333, 1), (45, 9000, 0)])]
+    single = []
+    for t in trajs:
+        body = eng.entropy(t, bins, "hist")
+        single.append((body.flat(), eng.mist(t.n_dih)[0]))
+    for _ in range(2):
+        bodies, trees = eng.entropy_batch(trajs, bins, "hist")
+        for (flat, edges), body, (e, _) in zip(single, bodies, trees):
+            assert np.array_equal(flat, body.flat()) and np.array_equal(edges, e)
