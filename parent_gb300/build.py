@@ -39,6 +39,7 @@ CU_SOURCES = {
     "pg_pairs_sorted.cu": [],
     "pg_pairs_onehot.cu": [],
     "pg_mist.cu": [],
+    "pg_mist_tree.cu": [],
     "pg_synth.cu": [],
     "pg_noalloc.cu": [],
     "pg_ingest.cu": [],
@@ -81,7 +82,7 @@ def build(verbose: bool = False, jobs: int | None = None) -> Path:
     BUILD.mkdir(exist_ok=True)
     LIBDIR.mkdir(exist_ok=True)
     BINDIR.mkdir(exist_ok=True)
-    headers = sorted(CSRC.glob("*.h")) + [INCLUDE / "parent_gb300.h", INCLUDE / "parent_gb300_io.h"]
+    headers = sorted(CSRC.glob("*.h")) + sorted(CSRC.glob("*.cuh")) + [INCLUDE / "parent_gb300.h", INCLUDE / "parent_gb300_io.h"]
     steps = []
     objs = []
     for src, extra in CU_SOURCES.items():

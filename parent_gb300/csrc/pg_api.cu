@@ -19,7 +19,7 @@ namespace pg {
 size_t prep_smem_bytes(const SysGeom &g);
 size_t mist_scratch_bytes(int D);
 cudaError_t launch_mist_impl(int D, int nb, int na, const double *mi, void *scratch,
-                             double *edge_mi, int *edge_from, int *edge_to, cudaStream_t st);
+                             double *edge_mi, int *edge_from, int *edge_to, const int *need, cudaStream_t st);
 bool synth_spec_ok(const pg_synth_spec *sp);
 size_t synth_scratch_bytes(const pg_synth_spec *sp, size_t *lat_bytes, size_t *sw_bytes,
                            std::vector<float> &lat, std::vector<int> &sw, std::vector<int> &sw_off);
@@ -123,6 +123,7 @@ struct pg_ctx {
     DevBuf batch, batchmeta, ohbatch;
     cudaGraphExec_t graph = nullptr;
     std::vector<int64_t> graph_key;
+    int graph_tree_launches = 0;
     // host trajectories: uploads run on their own stream, one event per DOF group
     cudaStream_t copy = nullptr;
     // pg_prefetch: the host columns of the next call, uploaded by the copy
@@ -1382,12 +1383,29 @@ PG_API int pg_mist(pg_ctx *ctx, int n_dihedrals, const pg_par_body *body, pg_mis
             return fail(ctx, PG_ERR_ARG, "no resident MI matrix for %d dihedrals", n_dihedrals);
     }
     CK(ctx->edges.ensure((size_t)D * (sizeof(double) + 2 * sizeof(int)) + 256));
-    CK(ctx->mistscr.ensure(mist_scratch_bytes(D)));
+    CK(ctx->mistscr.ensure(mist_tree_bytes(D) + mist_scratch_bytes(D)));
     double *emi = (double *)ctx->edges.p;
     int *efrom = (int *)(emi + D), *eto = efrom + D;
     CK(cudaEventRecord(ctx->ev[1], st));
-    CK(launch_mist_impl(D, nb, na, (const double *)ctx->mi.p, ctx->mistscr.p, emi, efrom, eto, st));
-    ctx->launches++;
+    {
+        MistDesc m{};
+        m.D = D;
+        m.nb = nb;
+        m.na = na;
+        m.mi = (const double *)ctx->mi.p;
+        m.scratch = ctx->mistscr.p;
+        m.prim = (char *)ctx->mistscr.p + mist_tree_bytes(D);
+        m.edge_mi = emi;
+        m.edge_from = efrom;
+        m.edge_to = eto;
+        int nl = 1;
+        if (mist_tree_supported(D)) {
+            m.need = (const int *)m.scratch;
+            CK(launch_mist_tree(nullptr, m, 1, D, st, &nl));
+        }
+        CK(launch_mist_impl(D, nb, na, m.mi, m.prim, emi, efrom, eto, m.need, st));
+        ctx->launches += nl;
+    }
     CK(cudaEventRecord(ctx->ev[2], st));
     // the 1D entropies (s1_b | s1_a | s1_d lead the body layout)
     CK(cudaMemcpyAsync(h_s1, body ? (const double *)ctx->par.p + L.s1b : dof_arrays(ctx, D).s1,
@@ -1674,7 +1692,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
             L.par = off;
             off = al256(off + (size_t)par_layout(g.n_dih).total * sizeof(double));
             L.mist = off;
-            off = al256(off + mist_scratch_bytes(g.D));
+            off = al256(off + mist_tree_bytes(g.D) + mist_scratch_bytes(g.D));
             L.edges = off;
             off = al256(off + (size_t)g.D * (sizeof(double) + 2 * sizeof(int)));
             if (g.sorted) {
@@ -1732,6 +1750,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
     auto dofs_at = [&](const BatchLayout &L) { return dof_at(arena + L.dof, L.g.D); };
     std::vector<SysDesc> sd((size_t)n_sys);
     std::vector<MistDesc> md((size_t)n_sys);
+    const bool tree = mist_tree_supported(maxD);
     std::vector<PairTile> tiles;
     std::vector<int> tsys;
     for (int s = 0; s < n_sys; s++) {
@@ -1750,6 +1769,8 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
         md[s].na = L.g.na;
         md[s].mi = (const double *)(arena + L.mi);
         md[s].scratch = arena + L.mist;
+        md[s].prim = arena + L.mist + mist_tree_bytes(L.g.D);
+        md[s].need = tree ? (const int *)md[s].scratch : nullptr;
         md[s].edge_mi = (double *)(arena + L.edges);
         md[s].edge_from = (int *)(md[s].edge_mi + L.g.D);
         md[s].edge_to = md[s].edge_from + L.g.D;
@@ -1857,6 +1878,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
     key.push_back(sys[0].g.ilv);
     key.push_back(onehot ? (int64_t)(uintptr_t)ctx->ohbatch.p : -1);
     key.push_back(srt ? (int64_t)(uintptr_t)ctx->sscr.p : -1);
+    key.push_back(tree);
     for (int k = 0; k < 6; k++) key.push_back(bins[k]);
     for (int s = 0; s < n_sys; s++) {
         const pg_bat_view &v = trajs[s];
@@ -1941,7 +1963,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
             e = cudaMemcpyAsync(arena + L.par, dofs_at(L).s1, (size_t)L.g.D * sizeof(double), cudaMemcpyDeviceToDevice,
                                 st);
         }
-        int oh_launches = 0;
+        int oh_launches = 0, tree_launches = 0;
         if (e == cudaSuccess && onehot)
             e = launch_pairs_onehot_batch(gs, ctx->ohbatch.p, (int *)ctx->errw.p, st, &oh_launches);
         else if (e == cudaSuccess && srt) {
@@ -1971,6 +1993,8 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
                                               (const int *)(meta + mo_ts), (int64_t)tiles.size(),
                                               (const unsigned long long *)ctx->nfix.p, ctx->nfix_scale,
                                               (int *)ctx->errw.p, T, st);
+        if (e == cudaSuccess && tree)
+            e = launch_mist_tree((const MistDesc *)(meta + mo_md), MistDesc{}, n_sys, maxD, st, &tree_launches);
         if (e == cudaSuccess) e = launch_mist_batch((const MistDesc *)(meta + mo_md), n_sys, maxD, st);
         cudaError_t e2 = cudaStreamEndCapture(st, &graph);
         if (e == cudaSuccess) e = e2;
@@ -1981,10 +2005,11 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
             return fail(ctx, PG_ERR_CUDA, "batch graph capture: %s", cudaGetErrorString(e));
         }
         ctx->graph_key = key;
+        ctx->graph_tree_launches = tree_launches;
     }
     CK(cudaGraphLaunch(ctx->graph, st));
     // preps, pair kernel (+ the one-hot finalize), MIST
-    ctx->launches += (pmap[0].empty() ? 0 : 1) + (pmap[1].empty() ? 0 : 1) + (onehot ? 3 : (srt ? 5 : 2));
+    ctx->launches += ctx->graph_tree_launches + (pmap[0].empty() ? 0 : 1) + (pmap[1].empty() ? 0 : 1) + (onehot ? 3 : (srt ? 5 : 2));
     CK(cudaEventRecord(ctx->ev[2], st));
     int rc = check_err_words(ctx);
     float ms[2];

@@ -379,16 +379,26 @@ cudaError_t prepare_pairs_onehot_batch(const std::vector<SysGeom> &gs, const std
 cudaError_t launch_pairs_onehot_batch(const std::vector<SysGeom> &gs, void *ws, int *err, cudaStream_t st,
                                       int *launches);
 
-// One system of a batched MIST launch (one CTA each); scratch holds
-// key[D] | from[D] | pos[D] (mist_scratch_bytes(D)).
+// One system of a MIST launch. scratch: mist_tree_bytes(D) for the tree
+// kernels; prim: mist_scratch_bytes(D) for the Prim kernels, which hold
+// key[D] | from[D] | pos[D] there; need: they run only if *need is not 0
+// (nullptr: always), the first word of scratch after the tree kernels.
 struct MistDesc {
     int D, nb, na;
     const double *mi;
-    void *scratch;
+    void *scratch, *prim;
+    const int *need;
     double *edge_mi;
     int *edge_from, *edge_to;
 };
 cudaError_t launch_mist_batch(const MistDesc *sys, int n_sys, int max_D, cudaStream_t st);
+// Boruvka's tree in the reference's order (pg_mist_tree.cu), for one system
+// (many == nullptr) or n_sys; sets the first word of a system's scratch where
+// the Prim kernels have to decide.
+bool mist_tree_supported(int max_D);
+size_t mist_tree_bytes(int D);
+cudaError_t launch_mist_tree(const MistDesc *many, const MistDesc &one, int n_sys, int max_D, cudaStream_t st,
+                             int *launches);
 
 // MI matrix from a .par body already on the device (get_mutual semantics).
 cudaError_t launch_mi_from_par(int n_dih, const double *par, ParLayout L, double *mi,

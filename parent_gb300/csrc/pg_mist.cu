@@ -32,6 +32,7 @@
 #include <stdlib.h>
 
 #include "pg_internal.h"
+#include "pg_okey.cuh"
 
 namespace pg {
 
@@ -39,19 +40,6 @@ namespace {
 
 constexpr int kMaxThreads = 1024;
 constexpr int kMaxWarps = kMaxThreads / 32;
-
-// order-preserving image of a double; 0 is below every value. NaN maps to 0:
-// it never beats anything, as no strict '>' with a NaN holds in the reference.
-__device__ __forceinline__ unsigned long long okey(double x) {
-    unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    if ((b & 0x7fffffffffffffffull) > 0x7ff0000000000000ull) return 0ull;  // NaN
-    if (b == 0x8000000000000000ull) b = 0ull;  // -0 == +0
-    return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
-}
-__device__ __forceinline__ double okey_value(unsigned long long k) {
-    const unsigned long long b = (k >> 63) ? (k & 0x7fffffffffffffffull) : ~k;
-    return __longlong_as_double((long long)b);
-}
 
 // A candidate: its key and a secondary word that orders equal keys,
 // ~((type(from) << 62) | (type(v) << 60) | (pos(from) << 30) | v), so that the
@@ -205,7 +193,8 @@ size_t mist_cluster_smem(int D) {
 
 __global__ void __launch_bounds__(kMaxThreads, 1)
 mist_cluster_kernel(int D, int nb, int na, const double *__restrict__ mi, double *edge_mi, int *edge_from,
-                    int *edge_to) {
+                    int *edge_to, const int *need) {
+    if (need && __ldg(need) == 0) return;
     extern __shared__ __align__(16) unsigned char smem[];
     const int S = (D + kClusterCtas - 1) / kClusterCtas;
     const int rank = (int)cluster_rank();
@@ -276,7 +265,8 @@ mist_cluster_kernel(int D, int nb, int na, const double *__restrict__ mi, double
 template <bool SMEM>
 __global__ void __launch_bounds__(kMaxThreads, 1)
 mist_kernel(int D, int nb, int na, const double *__restrict__ mi, unsigned long long *gkey, int *gfrom,
-            int *pos, double *edge_mi, int *edge_from, int *edge_to) {
+            int *pos, double *edge_mi, int *edge_from, int *edge_to, const int *need) {
+    if (need && __ldg(need) == 0) return;
     mist_body<SMEM>(D, nb, na, mi, gkey, gfrom, pos, edge_mi, edge_from, edge_to);
 }
 
@@ -284,7 +274,8 @@ mist_kernel(int D, int nb, int na, const double *__restrict__ mi, unsigned long 
 template <bool SMEM>
 __global__ void __launch_bounds__(kMaxThreads, 1) mist_batch_kernel(const MistDesc *__restrict__ sys) {
     const MistDesc &d = sys[blockIdx.x];
-    unsigned long long *gkey = (unsigned long long *)d.scratch;
+    if (d.need && __ldg(d.need) == 0) return;
+    unsigned long long *gkey = (unsigned long long *)d.prim;
     int *gfrom = (int *)(gkey + d.D);
     int *pos = gfrom + d.D;
     mist_body<SMEM>(d.D, d.nb, d.na, d.mi, gkey, gfrom, pos, d.edge_mi, d.edge_from, d.edge_to);
@@ -318,6 +309,7 @@ __global__ void mi_from_par_kernel(int n_dih, const double *par, ParLayout L, do
 
 size_t mist_scratch_bytes(int D) { return (size_t)D * (sizeof(double) + 2 * sizeof(int)) + 256; }
 
+// need: the kernel runs only if *need is not 0 when it starts (nullptr: always).
 // Prim over a cluster of 8 CTAs (kernel above) from kClusterMinD vertices up,
 // one CTA below; PG_MIST_CLUSTER=0 keeps one CTA.
 static bool mist_cluster_enabled() {
@@ -326,7 +318,7 @@ static bool mist_cluster_enabled() {
 }
 
 cudaError_t launch_mist_impl(int D, int nb, int na, const double *mi, void *scratch,
-                             double *edge_mi, int *edge_from, int *edge_to, cudaStream_t st) {
+                             double *edge_mi, int *edge_from, int *edge_to, const int *need, cudaStream_t st) {
     if (D >= kClusterMinD && mist_cluster_enabled()) {
         const size_t smem = mist_cluster_smem(D);
         if (smem <= 200 * 1024) {
@@ -345,7 +337,7 @@ cudaError_t launch_mist_impl(int D, int nb, int na, const double *mi, void *scra
             at[0].val.clusterDim.z = 1;
             cfg.attrs = at;
             cfg.numAttrs = 1;
-            e = cudaLaunchKernelEx(&cfg, kern, D, nb, na, mi, edge_mi, edge_from, edge_to);
+            e = cudaLaunchKernelEx(&cfg, kern, D, nb, na, mi, edge_mi, edge_from, edge_to, need);
             if (e != cudaSuccess) return e;
             return cudaGetLastError();
         }
@@ -359,9 +351,9 @@ cudaError_t launch_mist_impl(int D, int nb, int na, const double *mi, void *scra
         cudaError_t e = cudaFuncSetAttribute(mist_kernel<true>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        mist_kernel<true><<<1, nthr, smem, st>>>(D, nb, na, mi, gkey, gfrom, pos, edge_mi, edge_from, edge_to);
+        mist_kernel<true><<<1, nthr, smem, st>>>(D, nb, na, mi, gkey, gfrom, pos, edge_mi, edge_from, edge_to, need);
     } else {
-        mist_kernel<false><<<1, nthr, 0, st>>>(D, nb, na, mi, gkey, gfrom, pos, edge_mi, edge_from, edge_to);
+        mist_kernel<false><<<1, nthr, 0, st>>>(D, nb, na, mi, gkey, gfrom, pos, edge_mi, edge_from, edge_to, need);
     }
     return cudaGetLastError();
 }

@@ -1,0 +1,523 @@
+// MIST maximum spanning tree, found as a tree first and put into the
+// reference's order afterwards.
+//
+// Prim's algorithm (pg_mist.cu) takes D - 1 dependent steps over rows of the
+// MI matrix, 1.2 us each on one CTA, 2.4 to 3.7 us over a cluster. When the
+// tree is unique, the same edges come out of Boruvka's rounds (every component
+// takes its best outgoing edge at once, about log2(D) / 1.5 rounds, each a
+// parallel pass over the rows whose best neighbour has joined their own
+// component), and Prim's order of them needs only the tree: at every step the
+// best tree edge that leaves the part joined so far. The edges' ranks by MI
+// replace the values, the edges that leave the part are a bitmap over the
+// ranks, and a step is one warp's walk over a few words of shared memory.
+//
+// What makes this exact (get_PAR_MIST.cpp:441-748 keeps the first maximum in
+// its scan order): if every component's best outgoing edge is strictly better
+// than its other outgoing edges in every round, each of them is in every
+// maximum spanning tree, so the tree is unique; if all tree edges differ in MI
+// too, no step of Prim's has two best edges to choose from, and the order is
+// the values' alone. Any equality found on the way (and any row without a
+// comparable value: NaN) sets a flag; then the Prim kernels, which follow the
+// reference's tie order, run as before. Without the flag they return at once.
+//
+// Measured (kernels of one tree, against Prim's): see the launcher.
+#include <stdint.h>
+#include <stdlib.h>
+
+#include "pg_internal.h"
+#include "pg_okey.cuh"
+
+namespace pg {
+
+namespace {
+
+constexpr int kTie = 1 << 30;      // in bu: the row has its best value twice
+constexpr int kMergeThreads = 1024;
+constexpr int kScanWarps = 8;      // rows per CTA of a scan
+constexpr int kRankSplit = 8;      // CTAs sharing an edge's comparisons
+
+enum { CTL_FLAG = 0, CTL_NCOMP = 1, CTL_EDGES = 2 };
+
+// One system's working arrays, after the 256 bytes of ctl (and before the
+// Prim kernels' own scratch).
+struct Tree {
+    int D;
+    const double *mi;
+    int *ctl;
+    unsigned long long *bkey, *ckey, *ek, *ks;  // per vertex, per component, per edge, per rank
+    int *bu, *comp, *win, *parent, *ea, *eb, *rank, *seq;
+};
+
+__device__ __forceinline__ Tree tree_of(const MistDesc &d) {
+    Tree t;
+    t.D = d.D;
+    t.mi = d.mi;
+    t.ctl = (int *)d.scratch;
+    unsigned long long *p = (unsigned long long *)((char *)d.scratch + 256);
+    const size_t D = (size_t)d.D;
+    t.bkey = p;
+    t.ckey = p + D;
+    t.ek = p + 2 * D;
+    t.ks = p + 3 * D;
+    int *q = (int *)(p + 4 * D);
+    t.bu = q;
+    t.comp = q + D;
+    t.win = q + 2 * D;
+    t.parent = q + 3 * D;
+    t.ea = q + 4 * D;
+    t.eb = q + 5 * D;
+    t.rank = q + 6 * D;
+    t.seq = q + 7 * D;
+    return t;
+}
+
+__device__ __forceinline__ bool finished(const Tree &t) {
+    return __ldcg(t.ctl + CTL_FLAG) != 0 || __ldcg(t.ctl + CTL_NCOMP) <= 1;
+}
+
+// Row v's best neighbour outside its component, by one warp; a neighbour found
+// in an earlier round that is still outside is still the best one.
+__device__ __forceinline__ void scan_row(const Tree &t, int v, bool first, int lane) {
+    const int c = first ? v : t.comp[v];
+    if (!first) {
+        const int u = t.bu[v] & (kTie - 1);
+        if (t.bkey[v] && t.comp[u] != c) return;
+    }
+    unsigned long long best = 0ull;
+    int bu = 0;
+    bool tie = false;
+    const double *row = t.mi + (int64_t)v * t.D;
+    for (int u0 = lane; u0 < t.D; u0 += 128) {
+        double x[4];
+        int cu[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int u = u0 + 32 * j;
+            x[j] = u < t.D ? __ldg(row + u) : 0.0;
+            cu[j] = u < t.D ? (first ? u : t.comp[u]) : c;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (cu[j] == c) continue;
+            const unsigned long long k = okey(x[j]);
+            if (k > best) {
+                best = k;
+                bu = u0 + 32 * j;
+                tie = false;
+            } else if (k == best) {
+                tie = true;
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long k = __shfl_xor_sync(0xffffffffu, best, o);
+        const int u = __shfl_xor_sync(0xffffffffu, bu, o);
+        const bool ot = __shfl_xor_sync(0xffffffffu, (int)tie, o) != 0;
+        if (k > best) {
+            best = k;
+            bu = u;
+            tie = ot;
+        } else if (k == best) {
+            tie = tie || ot || u != bu;
+        }
+    }
+    if (lane == 0) {
+        t.bkey[v] = best;
+        t.bu[v] = bu | (tie ? kTie : 0);
+    }
+}
+
+// One round's unions, by one CTA: every component's best row, its edge, the
+// new components.
+__device__ __forceinline__ void merge_round(const Tree &t) {
+    const int tid = threadIdx.x, nthr = blockDim.x, D = t.D;
+    __shared__ int s_bad, s_more, s_roots;
+    if (tid == 0) s_bad = 0;
+    for (int v = tid; v < D; v += nthr) {
+        __stcg(t.ckey + v, 0ull);
+        __stcg(t.win + v, -1);
+    }
+    __syncthreads();
+    for (int v = tid; v < D; v += nthr) atomicMax(t.ckey + t.comp[v], t.bkey[v]);
+    __syncthreads();
+    for (int v = tid; v < D; v += nthr) {
+        const int c = t.comp[v];
+        const unsigned long long k = __ldcg(t.ckey + c);
+        if (k == 0ull) s_bad = 1;  // nothing comparable leaves the component
+        else if (t.bkey[v] == k && (atomicCAS(t.win + c, -1, v) != -1 || (t.bu[v] & kTie))) s_bad = 1;
+    }
+    __syncthreads();
+    if (s_bad) {
+        if (tid == 0) atomicExch(t.ctl + CTL_FLAG, 1);
+        return;
+    }
+    for (int c = tid; c < D; c += nthr) {
+        if (t.comp[c] != c) continue;  // roots carry their component's number
+        const int v = __ldcg(t.win + c), u = t.bu[v], c2 = t.comp[u], w = __ldcg(t.win + c2);
+        const bool mutual = w == u && t.bu[u] == v;  // the other component took the same edge
+        if (!mutual || c < c2) {
+            const int e = atomicAdd(t.ctl + CTL_EDGES, 1);
+            if (e < D - 1) {
+                t.ea[e] = v;
+                t.eb[e] = u;
+                t.ek[e] = t.bkey[v];
+            }
+        }
+        t.parent[c] = mutual && c < c2 ? c : c2;
+    }
+    __syncthreads();
+    for (int it = 0; it < 20; it++) {  // pointer doubling: at most log2(D) passes change anything
+        if (tid == 0) s_more = 0;
+        __syncthreads();
+        for (int c = tid; c < D; c += nthr) {
+            if (t.comp[c] != c) continue;
+            const int p = *(volatile int *)(t.parent + c), g = *(volatile int *)(t.parent + p);
+            if (g != p) {
+                *(volatile int *)(t.parent + c) = g;
+                s_more = 1;
+            }
+        }
+        __syncthreads();
+        const int more = s_more;
+        __syncthreads();
+        if (!more) break;
+    }
+    if (tid == 0) s_roots = 0;
+    __syncthreads();
+    int roots = 0;
+    for (int v = tid; v < D; v += nthr) {
+        const int c = t.comp[v], r = t.parent[c];
+        roots += v == c && r == c;
+        t.win[v] = r;  // the new number, copied once every old one has been read
+    }
+    if (roots) atomicAdd(&s_roots, roots);
+    __syncthreads();
+    for (int v = tid; v < D; v += nthr) t.comp[v] = t.win[v];
+    if (tid == 0) t.ctl[CTL_NCOMP] = s_roots;
+    __syncthreads();
+}
+
+// Edges better than edge e among [j0, j1), e's rank when summed over all edges
+__device__ __forceinline__ void rank_edge(const Tree &t, int e, int j0, int j1) {
+    const unsigned long long k = t.ek[e];
+    int n = 0;
+    bool same = false;
+    for (int j = j0; j < j1; j++) {
+        const unsigned long long x = t.ek[j];
+        n += x > k;
+        same = same || (x == k && j != e);
+    }
+    if (n) atomicAdd(t.rank + e, n);
+    if (same) atomicExch(t.ctl + CTL_FLAG, 1);
+}
+
+__host__ __device__ inline int pow2_above(int n) {
+    int p = 1;
+    while (p < n) p <<= 1;
+    return p;
+}
+// Bytes of order_tree's shared memory for D vertices: the adjacency starts
+// (then the parents) and, in turn, the arcs or the second tree with its keys.
+__host__ __device__ inline size_t order_smem(int D) {
+    const size_t n = (size_t)D + 4, second = n * 4 + n * 2 + (size_t)pow2_above(D) * 4;
+    return n * 4 + (n * 8 > second ? n * 8 : second);
+}
+
+// a[0 .. n) -> its inclusive sums, by the whole CTA (s_scan: 33 ints)
+__device__ __forceinline__ void cta_scan(int *a, int n, int *s_scan) {
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31;
+    const int per = (n + nthr - 1) / nthr, v0 = min(n, tid * per), v1 = min(n, v0 + per);
+    int s = 0;
+    for (int v = v0; v < v1; v++) s += a[v];
+    int x = s;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_scan[tid >> 5] = x;
+    __syncthreads();
+    if (tid < 32) {
+        int y = tid < (nthr >> 5) ? s_scan[tid] : 0;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int z = __shfl_up_sync(0xffffffffu, y, o);
+            if (lane >= o) y += z;
+        }
+        s_scan[tid + 1] = y;
+        if (tid == 0) s_scan[0] = 0;
+    }
+    __syncthreads();
+    int base = s_scan[tid >> 5] + x - s;
+    for (int v = v0; v < v1; v++) {
+        base += a[v];
+        a[v] = base;
+    }
+    __syncthreads();
+}
+
+// Prim's order of the tree's edges, without Prim's steps, by one CTA.
+//
+// Root the tree at bond 0 (In = {bond 0}, get_PAR_MIST.cpp:419-422). A vertex
+// u joins when the lightest edge of its path has been taken, then the lightest
+// edge of the rest of the path behind that one, and so on: the suffix minima
+// of the path's weights, the last of them u's own edge. Of two vertices the
+// one whose sequence has the heavier edge where they first differ joins first,
+// and a sequence comes before those it begins. So the joining order is the
+// preorder of a second tree, in which u hangs under the far end of the nearest
+// edge above its own that is lighter (under the root where none is), children
+// ordered by their edges from heavy to light (one sort by parent and rank):
+//   place(u) = sum over u and its ancestors a in that tree but the root of
+//              1 + sum of the subtree sizes of a's heavier siblings.
+// Rooting is an Euler tour ranked by pointer doubling; the walks up the two
+// trees are short in trees of data and at most D steps.
+__device__ __forceinline__ void order_tree(const Tree &t, double *edge_mi, int *edge_from, int *edge_to) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_scan[33];
+    __shared__ int s_more;
+    const int tid = threadIdx.x, nthr = blockDim.x, D = t.D, E = D - 1;
+    int *start = (int *)smem;                          // adjacency starts, D + 1
+    uint32_t *arc = (uint32_t *)(start + D + 4);        // 2 E arcs: next | distance to it << 16
+    int *sa = t.win, *sb = t.seq;                       // an edge's two arcs: a -> b in a's list, b -> a in b's
+    constexpr uint32_t kEnd = 0xffffu;
+    for (int k = tid; k < D + 1; k += nthr) start[k] = 0;
+    __syncthreads();
+    for (int e = tid; e < E; e += nthr) {
+        t.ks[__ldcg(t.rank + e)] = t.ek[e];
+        atomicAdd(&start[t.ea[e]], 1);
+        atomicAdd(&start[t.eb[e]], 1);
+    }
+    __syncthreads();
+    cta_scan(start, D, s_scan);  // the lists' ends: filled downwards
+    if (tid == 0) start[D] = 2 * E;
+    __syncthreads();
+    for (int e = tid; e < E; e += nthr) {
+        sa[e] = atomicSub(&start[t.ea[e]], 1) - 1;
+        sb[e] = atomicSub(&start[t.eb[e]], 1) - 1;
+    }
+    __syncthreads();
+    // after an arc into a vertex comes the one after its reverse in that
+    // vertex's list; the arc that would come back to the first one ends the tour
+    const int first = start[0];
+    for (int e = tid; e < E; e += nthr) {
+        const int a = t.ea[e], b = t.eb[e], ia = sa[e], ib = sb[e];
+        const int na = ib + 1 < start[b + 1] ? ib + 1 : start[b], nb = ia + 1 < start[a + 1] ? ia + 1 : start[a];
+        arc[ia] = na == first ? kEnd : (uint32_t)na | 1u << 16;
+        arc[ib] = nb == first ? kEnd : (uint32_t)nb | 1u << 16;
+    }
+    __syncthreads();
+    for (int it = 0; it < 20; it++) {
+        if (tid == 0) s_more = 0;
+        __syncthreads();
+        for (int k = tid; k < 2 * E; k += nthr) {
+            // next and distance in one word: a neighbour's pair is consistent
+            // whether or not it has moved on in this pass
+            const uint32_t x = *(volatile uint32_t *)(arc + k);
+            if ((x & 0xffffu) == kEnd) continue;
+            const uint32_t y = *(volatile uint32_t *)(arc + (x & 0xffffu));
+            *(volatile uint32_t *)(arc + k) = (y & 0xffffu) | ((x & 0xffff0000u) + (y & 0xffff0000u));
+            if ((y & 0xffffu) != kEnd) s_more = 1;
+        }
+        __syncthreads();
+        const int more = s_more;
+        __syncthreads();
+        if (!more) break;
+    }
+    uint32_t *up = (uint32_t *)start;  // a vertex's parent | its edge's rank << 16 (rank 0: the heaviest)
+    for (int e = tid; e < E; e += nthr) {
+        const int a = t.ea[e], b = t.eb[e];
+        const bool down = (arc[sa[e]] >> 16) > (arc[sb[e]] >> 16);  // a -> b comes first
+        // start is not read any more by anyone past the barrier above
+        up[down ? b : a] = (uint32_t)(down ? a : b) | (uint32_t)__ldcg(t.rank + e) << 16;
+    }
+    __syncthreads();
+    int *size = (int *)arc;                          // subtree sizes, then the sums' terms, D
+    uint16_t *over = (uint16_t *)(size + D + 4);     // parent in the second tree, D
+    uint32_t *key = (uint32_t *)(over + D + (D & 1));
+    const int n2 = pow2_above(E);
+    for (int u = tid; u < D; u += nthr) size[u] = 1;
+    for (int u = 1 + tid; u < D; u += nthr) {
+        const uint32_t me = up[u];
+        uint32_t a = me & 0xffffu;
+        while (a != 0u) {
+            const uint32_t x = up[a];
+            if ((x >> 16) > (me >> 16)) break;  // a lighter edge
+            a = x & 0xffffu;
+        }
+        over[u] = (uint16_t)a;
+        t.bu[me >> 16] = u;  // the vertex of a rank
+    }
+    __syncthreads();
+    for (int u = 1 + tid; u < D; u += nthr)
+        for (uint32_t a = over[u]; a != 0u; a = over[a]) atomicAdd(&size[a], 1);
+    // siblings together, heavy to light: sorted by (parent, rank)
+    for (int k = tid; k < n2; k += nthr) key[k] = k < E ? (uint32_t)over[k + 1] << 16 | up[k + 1] >> 16 : 0xffffffffu;
+    __syncthreads();
+    for (int k = 2; k <= n2; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int q = tid; q < n2 / 2; q += nthr) {
+                const int i = ((q & ~(j - 1)) << 1) | (q & (j - 1));
+                const uint32_t x = key[i], y = key[i | j];
+                if ((x > y) == ((i & k) == 0)) {
+                    key[i] = y;
+                    key[i | j] = x;
+                }
+            }
+            __syncthreads();
+        }
+    int *sum = t.parent, *term = t.comp;
+    for (int k = tid; k < E; k += nthr) sum[k] = size[t.bu[key[k] & 0xffffu]];
+    __syncthreads();
+    cta_scan(sum, E, s_scan);
+    for (int k = tid; k < E; k += nthr) {
+        const uint32_t x = key[k];
+        int lo = 0, hi = k;  // the first sibling
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (key[mid] >> 16 < x >> 16) lo = mid + 1;
+            else hi = mid;
+        }
+        term[t.bu[x & 0xffffu]] = 1 + (k > 0 ? sum[k - 1] : 0) - (lo > 0 ? sum[lo - 1] : 0);
+    }
+    __syncthreads();
+    for (int u = 1 + tid; u < D; u += nthr) size[u] = term[u];
+    __syncthreads();
+    for (int u = 1 + tid; u < D; u += nthr) {
+        int step = -1;
+        for (uint32_t a = u; a != 0u; a = over[a]) step += size[a];
+        const uint32_t me = up[u];
+        edge_mi[step] = okey_value(t.ks[me >> 16]);
+        edge_from[step] = (int)(me & 0xffffu);
+        edge_to[step] = u;
+    }
+}
+
+__device__ __forceinline__ MistDesc sys_of(const MistDesc *many, const MistDesc &one, int s) { return many ? many[s] : one; }
+
+__device__ __forceinline__ void init_tree(const Tree &t, int i0, int stride) {
+    for (int v = i0; v < t.D; v += stride) {
+        t.comp[v] = v;
+        t.rank[v] = 0;
+    }
+    if (i0 == 0) {
+        t.ctl[CTL_FLAG] = 0;
+        t.ctl[CTL_NCOMP] = t.D;
+        t.ctl[CTL_EDGES] = 0;
+    }
+}
+
+__global__ void __launch_bounds__(256) tree_init_kernel(const MistDesc *many, const __grid_constant__ MistDesc one) {
+    const Tree t = tree_of(sys_of(many, one, blockIdx.y));
+    init_tree(t, blockIdx.x * 256 + threadIdx.x, gridDim.x * 256);
+}
+
+__global__ void __launch_bounds__(kScanWarps * 32)
+tree_scan_kernel(const MistDesc *many, const __grid_constant__ MistDesc one, int first) {
+    const Tree t = tree_of(sys_of(many, one, blockIdx.y));
+    const int v = blockIdx.x * kScanWarps + (threadIdx.x >> 5);
+    if (v >= t.D || finished(t)) return;
+    scan_row(t, v, first != 0, threadIdx.x & 31);
+}
+
+__global__ void __launch_bounds__(kMergeThreads)
+tree_merge_kernel(const MistDesc *many, const __grid_constant__ MistDesc one) {
+    const Tree t = tree_of(sys_of(many, one, blockIdx.x));
+    if (finished(t)) return;
+    merge_round(t);
+}
+
+__global__ void __launch_bounds__(256) tree_rank_kernel(const MistDesc *many, const __grid_constant__ MistDesc one) {
+    const Tree t = tree_of(sys_of(many, one, blockIdx.z));
+    const int e = blockIdx.x * 256 + threadIdx.x, E = t.D - 1;
+    if (e >= E || __ldcg(t.ctl + CTL_NCOMP) != 1) return;
+    const int per = (E + kRankSplit - 1) / kRankSplit, j0 = min(E, (int)blockIdx.y * per);
+    rank_edge(t, e, j0, min(E, j0 + per));
+}
+
+__global__ void __launch_bounds__(kMergeThreads)
+tree_order_kernel(const MistDesc *many, const __grid_constant__ MistDesc one) {
+    const MistDesc d = sys_of(many, one, blockIdx.x);
+    const Tree t = tree_of(d);
+    // not one component, or not D - 1 edges: the Prim kernels take over
+    const bool whole = __ldcg(t.ctl + CTL_NCOMP) == 1 && __ldcg(t.ctl + CTL_EDGES) == t.D - 1;
+    if (!whole || __ldcg(t.ctl + CTL_FLAG)) {
+        if (threadIdx.x == 0) atomicExch(t.ctl + CTL_FLAG, 1);
+        return;
+    }
+    order_tree(t, d.edge_mi, d.edge_from, d.edge_to);
+}
+
+// Everything in one CTA per system.
+__global__ void __launch_bounds__(kMergeThreads)
+tree_small_kernel(const MistDesc *many, const __grid_constant__ MistDesc one) {
+    const MistDesc d = sys_of(many, one, blockIdx.x);
+    const Tree t = tree_of(d);
+    const int tid = threadIdx.x;
+    init_tree(t, tid, kMergeThreads);
+    __syncthreads();
+    for (int round = 0; round < 32; round++) {
+        for (int v = tid >> 5; v < t.D; v += kMergeThreads / 32) scan_row(t, v, round == 0, tid & 31);
+        __syncthreads();
+        merge_round(t);
+        __syncthreads();
+        if (finished(t)) break;  // the same for every thread: written before the barrier
+    }
+    const int E = t.D - 1;
+    __syncthreads();
+    if (__ldcg(t.ctl + CTL_FLAG) == 0 && __ldcg(t.ctl + CTL_NCOMP) == 1)
+        for (int e = tid; e < E; e += kMergeThreads) rank_edge(t, e, 0, E);
+    __syncthreads();
+    const bool whole = __ldcg(t.ctl + CTL_NCOMP) == 1 && __ldcg(t.ctl + CTL_EDGES) == E;
+    if (!whole || __ldcg(t.ctl + CTL_FLAG)) {
+        if (tid == 0) atomicExch(t.ctl + CTL_FLAG, 1);
+        return;
+    }
+    __syncthreads();
+    order_tree(t, d.edge_mi, d.edge_from, d.edge_to);
+}
+
+// One CTA to 256 vertices (144: 0.074 ms, 0.107 over the grid; 294: 0.138 and
+// 0.126).
+constexpr int kSmallD = 256;
+constexpr int kTreeMaxD = 16000;  // order_smem within a CTA's shared memory; arcs and distances in 16 bits
+
+}  // namespace
+
+// From 40 vertices on (18: 0.033 ms against Prim's 0.023, 66: 0.046 and 0.072).
+bool mist_tree_supported(int max_D) {
+    if (getenv("PG_MIST_CLUSTER")) return false;  // a choice among the Prim kernels
+    return max_D >= 40 && max_D <= kTreeMaxD;
+}
+
+size_t mist_tree_bytes(int D) { return 256 + (size_t)D * (4 * sizeof(unsigned long long) + 8 * sizeof(int)); }
+
+// All kernels of one tree, Prim's before: 294 DOFs 0.36 -> 0.13 ms, 603 0.92 ->
+// 0.15, 2,994 6.97 -> 0.33, 7,494 27.9 -> 0.86, 14,994 67.4 -> 2.1. At 7,494:
+// four scans 0.42 ms (450 MB of MI each, 3.6 TB/s), their unions 0.15, the
+// ranks 0.04, the order 0.15, rounds that find nothing left 0.08.
+cudaError_t launch_mist_tree(const MistDesc *many, const MistDesc &one, int n_sys, int max_D, cudaStream_t st,
+                             int *launches) {
+    const size_t smem = order_smem(max_D);
+    if (max_D <= kSmallD) {
+        cudaError_t e = cudaFuncSetAttribute(tree_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        tree_small_kernel<<<n_sys, kMergeThreads, smem, st>>>(many, one);
+        *launches += 1;
+        return cudaGetLastError();
+    }
+    cudaError_t e = cudaFuncSetAttribute(tree_order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const unsigned n = (unsigned)n_sys;
+    tree_init_kernel<<<dim3((unsigned)((max_D + 255) / 256), n), 256, 0, st>>>(many, one);
+    int rounds = 0;
+    while ((1 << rounds) < max_D) rounds++;  // the components at least halve; the rounds left over return at once
+    for (int r = 0; r < rounds; r++) {
+        tree_scan_kernel<<<dim3((unsigned)((max_D + kScanWarps - 1) / kScanWarps), n), kScanWarps * 32, 0, st>>>(many, one,
+                                                                                                             r == 0);
+        tree_merge_kernel<<<n, kMergeThreads, 0, st>>>(many, one);
+    }
+    tree_rank_kernel<<<dim3((unsigned)((max_D + 255) / 256), kRankSplit, n), 256, 0, st>>>(many, one);
+    tree_order_kernel<<<n, kMergeThreads, smem, st>>>(many, one);
+    *launches += 3 + 2 * rounds;
+    return cudaGetLastError();
+}
+
+}  // namespace pg

@@ -18,7 +18,7 @@
 
 namespace pg {
 cudaError_t launch_mist_impl(int D, int nb, int na, const double *mi, void *scratch,
-                             double *edge_mi, int *edge_from, int *edge_to, cudaStream_t st);
+                             double *edge_mi, int *edge_from, int *edge_to, const int *need, cudaStream_t st);
 size_t mist_scratch_bytes(int D);
 void set_global_error(const char *msg);
 }  // namespace pg
@@ -82,7 +82,7 @@ extern "C" PG_API int pg_mist_noalloc(int n_dihedrals, const double *mi, double 
     // key/from entry it reads and writes each insertion position before
     // reading it, so leftover contents of an earlier call need no clearing.
     const int nb = n_dihedrals + 2, na = n_dihedrals + 1;
-    cudaError_t e = pg::launch_mist_impl((int)D, nb, na, mi, scratch, edge_mi, edge_from, edge_to,
+    cudaError_t e = pg::launch_mist_impl((int)D, nb, na, mi, scratch, edge_mi, edge_from, edge_to, nullptr,
                                          (cudaStream_t)stream);
     if (e != cudaSuccess) {
         pg::set_global_error(cudaGetErrorString(e));

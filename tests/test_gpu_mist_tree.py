@@ -1,0 +1,97 @@
+"""The tree kernels of the MIST (pg_mist_tree.cu): the edges, their order and
+their MI are the oracle's and the Prim kernels' exactly, for trees of every
+shape (the order is derived from the tree alone) and around the sizes where
+the kernels change; where MI values are equal or not comparable the Prim
+kernels decide, and the results are theirs."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import oracle
+import parent_gb300 as pg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def eng():
+    e = pg.Engine(0)
+    yield e
+    e.close()
+
+
+def _body(n_dih: int, mi: np.ndarray) -> pg.ParBody:
+    """A body with S1 = 0 whose mutual informations are mi exactly (S2 = -MI)."""
+    lo, n = {"b": 0, "a": n_dih + 2, "d": 2 * n_dih + 3}, {"b": n_dih + 2, "a": n_dih + 1, "d": n_dih}
+    body = pg.ParBody.empty(n_dih)
+    for p in ("bb", "ba", "bd", "aa", "ad", "dd"):
+        q = -mi[lo[p[0]]:lo[p[0]] + n[p[0]], lo[p[1]]:lo[p[1]] + n[p[1]]]
+        body.blocks[p][:] = q[np.triu_indices(n[p[0]], 1)][::-1] if p[0] == p[1] else q.reshape(-1)
+    return body
+
+
+def _mi(shape: str, D: int, seed: int) -> np.ndarray:
+    rng = np.random.default_rng(seed)
+    m = rng.random((D, D)) * 0.5
+    perm = rng.permutation(D)
+    perm = np.concatenate([[0], perm[perm != 0]])  # the root first
+    w = 1.0 + rng.random(D)
+    if shape == "falling chain":
+        w = 3.0 - np.arange(D) / D
+    if shape == "rising chain":
+        w = 1.0 + np.arange(D) / D
+    for k in range(1, D):
+        up = {"star": 0, "random": rng.integers(0, k)}.get(shape, k - 1)
+        m[perm[k], perm[up]] = m[perm[up], perm[k]] = w[k]
+    m = np.triu(m, 1)
+    return m + m.T
+
+
+@pytest.mark.parametrize("shape", ["random", "falling chain", "rising chain", "star", "zigzag chain", "no tree"])
+@pytest.mark.parametrize("n_dih", [13, 84, 85, 300])  # 42, 255, 258 and 903 DOFs: one CTA and the grid
+def test_tree_order_matches_oracle_and_prim(eng, monkeypatch, n_dih, shape):
+    D = 3 * n_dih + 3
+    m = _mi(shape, D, D) if shape != "no tree" else np.random.default_rng(D).normal(size=(D, D))
+    if shape == "no tree":
+        m = np.triu(m, 1) + np.triu(m, 1).T
+    body = _body(n_dih, m)
+    e, t = eng.mist(n_dih, body)
+    re, rt = oracle.mist(n_dih, body.blocks)
+    for f in ("t1", "t2", "i1", "i2", "left", "mi"):
+        assert np.array_equal(e[f], re[f]), f
+    monkeypatch.setenv("PG_MIST_CLUSTER", "1")
+    pe, pt = eng.mist(n_dih, body)
+    assert np.array_equal(e, pe) and np.array_equal(t, pt)
+
+
+@pytest.mark.parametrize("n_dih", [20, 150])
+@pytest.mark.parametrize("kind", ["two equal edges", "quantised", "all equal", "nan", "nan row"])
+def test_ties_and_nan_are_prims(eng, monkeypatch, n_dih, kind):
+    D = 3 * n_dih + 3
+    m = _mi("random", D, 7)
+    if kind == "two equal edges":  # the two heaviest of the whole matrix, not adjacent
+        m[3, 9] = m[9, 3] = m[20, 40] = m[40, 20] = 5.0
+    if kind == "quantised":
+        m = np.round(m * 8) / 8
+    if kind == "all equal":
+        m[:] = 0.25
+    if kind == "nan":
+        m[5, 17] = m[17, 5] = np.nan
+    if kind == "nan row":
+        m[:, 11] = m[11, :] = np.nan
+    body = _body(n_dih, m)
+    if kind == "nan row":  # no edge reaches this DOF: an error, as from the Prim kernels
+        with pytest.raises(pg.PGError) as new:
+            eng.mist(n_dih, body)
+        monkeypatch.setenv("PG_MIST_CLUSTER", "1")
+        with pytest.raises(pg.PGError) as old:
+            eng.mist(n_dih, body)
+        assert str(new.value) == str(old.value)
+        return
+    e, t = eng.mist(n_dih, body)
+    monkeypatch.setenv("PG_MIST_CLUSTER", "1")
+    pe, pt = eng.mist(n_dih, body)
+    for f in e.dtype.names:
+        assert np.array_equal(e[f], pe[f], equal_nan=f == "mi"), f
+    assert np.array_equal(t, pt, equal_nan=True)
