@@ -110,10 +110,12 @@ struct DofArrays {
                              // per-DOF constant of the 2D entropy decomposition
     int *b2;                 // 2D bin count of the DOF's type
     int *m2;                 // largest marginal count over the DOF's 2D bins
+    int *h2;                 // the marginal counts, kSegLd per DOF
 };
 
 // One system's DofArrays in one allocation of dof_bytes(D) bytes at base
-inline size_t dof_bytes(int D) { return (size_t)D * (5 * sizeof(double) + 2 * sizeof(int)) + 64; }
+constexpr int kSegLd = 220;  // ints per DOF of marginal counts or list segment starts (at most 218 bins, and the end)
+inline size_t dof_bytes(int D) { return (size_t)D * (5 * sizeof(double) + (2 + kSegLd) * sizeof(int)) + 64; }
 inline DofArrays dof_at(void *base, int D) {
     DofArrays d;
     double *b = (double *)base;
@@ -124,6 +126,7 @@ inline DofArrays dof_at(void *base, int D) {
     d.acon = b + 4 * (size_t)D;
     d.b2 = (int *)(b + 5 * (size_t)D);
     d.m2 = d.b2 + D;
+    d.h2 = d.m2 + D;
     return d;
 }
 
@@ -256,7 +259,6 @@ cudaError_t launch_pairs_hist32_batch(int bmax, bool codes, bool ilv, const SysD
 // (after the preprocessing), then per batch of rows launch_sorted_lists and
 // launch_pairs_sorted (which adds to the zeroed MI matrix's storage), then
 // launch_sorted_finish (S2D into the body, MI in place of the sums).
-constexpr int kSegLd = 220;  // ints per row of segment starts (at most 218 bins, and the end)
 struct SortedItem {          // segments of share `part` of row x column block
     int sys, row, blk, part;
 };

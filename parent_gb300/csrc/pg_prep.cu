@@ -436,6 +436,7 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
         unsigned int s = 0;
         for (int w = 0; w < copies; w++) s += h[w * stride + kk];
         h[kk] = s;
+        if (k >= B1) dof.h2[(int64_t)g * kSegLd + kk] = (int)s;
     }
     __syncthreads();
 
