@@ -180,7 +180,11 @@ class ParBody:
 
     @classmethod
     def empty(cls, n_dih: int) -> "ParBody":
-        return cls(n_dih, {k: np.zeros(n, dtype=np.float64) for k, n in block_sizes(n_dih).items()})
+        # one array: its blocks come back in one copy
+        sizes = block_sizes(n_dih)
+        at = np.cumsum([0] + list(sizes.values()))
+        flat = np.zeros(at[-1], dtype=np.float64)
+        return cls(n_dih, {k: flat[o:o + n] for (k, n), o in zip(sizes.items(), at)})
 
     def c(self) -> ParBodyC:
         b = ParBodyC()

@@ -373,28 +373,57 @@ static int run_prep(pg_ctx *ctx, const pg_bat_view *tv, const int bins[6], int f
     return PG_OK;
 }
 
+// The runs of a .par body's non-empty blocks that follow each other in the
+// caller's memory, each as one copy: copy(offset in the body, first block's
+// pointer, doubles). A copy costs several microseconds whatever its size, and
+// a body in one array is nine of them. Blocks are joined in ordinary host
+// memory only: neighbouring pinned or device allocations are not one range to
+// the runtime. A missing block ends the walk with its number, else -1.
+template <typename Ptr, typename Copy>
+static int body_runs(Ptr *const blk[9], const ParLayout &L, Copy &&copy) {
+    const int64_t off[10] = {L.s1b, L.s1a, L.s1d, L.bb, L.ba, L.bd, L.aa, L.ad, L.dd, L.total};
+    for (int k = 0; k < 9; k++)
+        if (off[k + 1] > off[k] && !blk[k]) return k;
+    auto plain = [](const void *p) {
+        cudaPointerAttributes at{};
+        return cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
+    };
+    for (int k = 0; k < 9;) {
+        int64_t n = off[k + 1] - off[k];
+        int j = k + 1;
+        for (; n > 0 && j < 9; j++) {
+            const int64_t m = off[j + 1] - off[j];
+            if (m > 0 && (blk[j] != blk[k] + n || !plain(blk[k]) || !plain(blk[j]))) break;
+            n += m;
+        }
+        if (n > 0) copy(off[k], blk[k], n);
+        k = j;
+    }
+    return -1;
+}
+
 // Enqueues the copies of a device .par body (layout L) into the caller's
 // blocks (host memory, or device memory of this context's GPU: the copy
 // direction comes from the pointers); every non-empty block needs a
 // destination.
 static int body_to_host(pg_ctx *ctx, const double *par, const ParLayout &L, const pg_par_body *out, int sys) {
     double *dst[9] = {out->s1_b, out->s1_a, out->s1_d, out->bb, out->ba, out->bd, out->aa, out->ad, out->dd};
-    const int64_t off[10] = {L.s1b, L.s1a, L.s1d, L.bb, L.ba, L.bd, L.aa, L.ad, L.dd, L.total};
-    for (int k = 0; k < 9; k++) {
-        const int64_t n = off[k + 1] - off[k];
-        if (n <= 0) continue;
-        if (!dst[k]) {
-            if (sys >= 0) return fail(ctx, PG_ERR_ARG, "system %d: null output block %d", sys, k);
-            return fail(ctx, PG_ERR_ARG, "null output block %d", k);
-        }
-        CK(cudaMemcpyAsync(dst[k], par + off[k], (size_t)n * sizeof(double), cudaMemcpyDefault, ctx->stream));
+    cudaError_t e = cudaSuccess;
+    const int k = body_runs(dst, L, [&](int64_t o, double *p, int64_t n) {
+        if (e == cudaSuccess) e = cudaMemcpyAsync(p, par + o, (size_t)n * sizeof(double), cudaMemcpyDefault, ctx->stream);
+    });
+    if (k >= 0) {
+        if (sys >= 0) return fail(ctx, PG_ERR_ARG, "system %d: null output block %d", sys, k);
+        return fail(ctx, PG_ERR_ARG, "null output block %d", k);
     }
+    CK(e);
     return PG_OK;
 }
 
 static int check_err_words(pg_ctx *ctx) {
-    int h[ERR_WORDS];
-    CK(cudaMemcpyAsync(h, ctx->errw.p, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(ctx->ensure_hstage(ERR_WORDS * sizeof(int)));
+    const int *h = (const int *)ctx->hstage;
+    CK(cudaMemcpyAsync(ctx->hstage, ctx->errw.p, ERR_WORDS * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (h[ERR_NEG_BOND]) return fail(ctx, PG_ERR_DATA, "ERROR: %d bond(s) smaller than 0.0", h[ERR_NEG_BOND]);
     if (h[ERR_MODFIT_RANGE])
@@ -1363,18 +1392,17 @@ PG_API int pg_mist(pg_ctx *ctx, int n_dihedrals, const pg_par_body *body, pg_mis
     int *hf = (int *)(hmi + D), *ht = hf + D;
     CK(cudaEventRecord(ctx->ev[0], st));
     if (body) {
-        const double *src[9] = {body->s1_b, body->s1_a, body->s1_d, body->bb, body->ba, body->bd, body->aa, body->ad, body->dd};
-        const int64_t off[10] = {L.s1b, L.s1a, L.s1d, L.bb, L.ba, L.bd, L.aa, L.ad, L.dd, L.total};
+        double *src[9] = {body->s1_b, body->s1_a, body->s1_d, body->bb, body->ba, body->bd, body->aa, body->ad, body->dd};
         CK(ctx->par.ensure((size_t)L.total * sizeof(double)));
         CK(ctx->mi.ensure((size_t)D * D * sizeof(double)));
-        for (int k = 0; k < 9; k++) {
-            const int64_t n = off[k + 1] - off[k];
-            if (n <= 0) continue;
-            if (!src[k]) return fail(ctx, PG_ERR_ARG, "null body block %d", k);
+        cudaError_t e = cudaSuccess;
+        const int k = body_runs(src, L, [&](int64_t o, double *p, int64_t n) {
             // host or device blocks: the copy direction comes from the pointers
-            CK(cudaMemcpyAsync((double *)ctx->par.p + off[k], src[k], (size_t)n * sizeof(double), cudaMemcpyDefault,
-                               st));
-        }
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync((double *)ctx->par.p + o, p, (size_t)n * sizeof(double), cudaMemcpyDefault, st);
+        });
+        if (k >= 0) return fail(ctx, PG_ERR_ARG, "null body block %d", k);
+        CK(e);
         CK(launch_mi_from_par(n_dihedrals, (const double *)ctx->par.p, L, (double *)ctx->mi.p, st));
         ctx->launches++;
         ctx->resident = false;
@@ -1410,11 +1438,9 @@ PG_API int pg_mist(pg_ctx *ctx, int n_dihedrals, const pg_par_body *body, pg_mis
     // the 1D entropies (s1_b | s1_a | s1_d lead the body layout)
     CK(cudaMemcpyAsync(h_s1, body ? (const double *)ctx->par.p + L.s1b : dof_arrays(ctx, D).s1,
                        (size_t)D * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (D > 1) {
-        CK(cudaMemcpyAsync(hmi, emi, (size_t)(D - 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(hf, efrom, (size_t)(D - 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(ht, eto, (size_t)(D - 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
-    }
+    // MI | from | to of D steps each lie one after the other on both sides
+    if (D > 1)
+        CK(cudaMemcpyAsync(hmi, emi, (size_t)D * (sizeof(double) + 2 * sizeof(int)), cudaMemcpyDeviceToHost, st));
     CK(cudaEventRecord(ctx->ev[3], st));
     CK(cudaStreamSynchronize(st));
     memcpy(s1.data(), h_s1, (size_t)D * sizeof(double));
@@ -2023,35 +2049,39 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
     if (rc) return rc;
     ctx->last_form = onehot ? PG_FORM_ONEHOT : PG_FORM_HIST;
 
-    // ---- results to the caller
-    for (int s = 0; s < n_sys; s++) {
-        const BatchLayout &L = sys[s];
-        const ParLayout PL = par_layout(L.g.n_dih);
-        if (outs) {
-            const int rcb = body_to_host(ctx, (const double *)(arena + L.par), PL, &outs[s], s);
-            if (rcb) return rcb;
-        }
-        if ((edges && edges[s]) || totals) {
-            const int D = L.g.D;
-            std::vector<double> hmi((size_t)D), s1((size_t)D);
-            std::vector<int> hf((size_t)D), ht((size_t)D);
-            const double *emi = (const double *)(arena + L.edges);
-            const int *ef = (const int *)(emi + D), *et = ef + D;
-            if (D > 1) {
-                CK(cudaMemcpyAsync(hmi.data(), emi, (size_t)(D - 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
-                CK(cudaMemcpyAsync(hf.data(), ef, (size_t)(D - 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
-                CK(cudaMemcpyAsync(ht.data(), et, (size_t)(D - 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
-            }
-            CK(cudaMemcpyAsync(s1.data(), (const double *)(arena + L.par), (size_t)D * sizeof(double),
+    // ---- results to the caller: the trees of all systems through pinned
+    // memory with one wait, then the bodies
+    const bool want_trees = edges || totals;
+    size_t rows = 0;  // of all systems: S1, then MI | from | to of each one's steps
+    for (const BatchLayout &L : sys) rows += (size_t)L.g.D;
+    if (want_trees) {
+        CK(ctx->ensure_hstage(rows * (2 * sizeof(double) + 2 * sizeof(int))));
+        char *h = (char *)ctx->hstage;
+        for (const BatchLayout &L : sys) {
+            const size_t D = (size_t)L.g.D;
+            CK(cudaMemcpyAsync(h, arena + L.par, D * sizeof(double), cudaMemcpyDeviceToHost, st));
+            CK(cudaMemcpyAsync(h + D * sizeof(double), arena + L.edges, D * (sizeof(double) + 2 * sizeof(int)),
                                cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            std::vector<pg_mist_edge> tmp((size_t)std::max(D - 1, 1));
+            h += D * (2 * sizeof(double) + 2 * sizeof(int));
+        }
+        CK(cudaStreamSynchronize(st));
+        h = (char *)ctx->hstage;
+        for (int s = 0; s < n_sys; s++) {
+            const size_t D = (size_t)sys[s].g.D;
+            const double *s1 = (const double *)h, *hmi = s1 + D;
+            const int *hf = (const int *)(hmi + D);
+            h += D * (2 * sizeof(double) + 2 * sizeof(int));
+            if (!((edges && edges[s]) || totals)) continue;
+            std::vector<pg_mist_edge> tmp(edges && edges[s] ? 0 : D);
             double tt[10];
-            pg_mist_edge *e = (edges && edges[s]) ? edges[s] : tmp.data();
-            rc = mist_edges_to_user(ctx, L.g.n_dih, hmi.data(), hf.data(), ht.data(), s1.data(), e, tt);
+            rc = mist_edges_to_user(ctx, sys[s].g.n_dih, hmi, hf, hf + D, s1, tmp.empty() ? edges[s] : tmp.data(), tt);
             if (rc) return rc;
             if (totals) memcpy(totals + 10 * (size_t)s, tt, sizeof tt);
         }
+    }
+    for (int s = 0; outs && s < n_sys; s++) {
+        const int rcb = body_to_host(ctx, (const double *)(arena + sys[s].par), par_layout(sys[s].g.n_dih), &outs[s], s);
+        if (rcb) return rcb;
     }
     CK(cudaStreamSynchronize(st));
     return PG_OK;
