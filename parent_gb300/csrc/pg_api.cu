@@ -571,7 +571,8 @@ static int run_sorted(pg_ctx *ctx, const SysGeom &g, const DofArrays &dof, const
     d.seg = (int *)(d.list + (size_t)rows * ld);
     d.list_ld = ld;
     d.pad = sorted_pad(g.D);
-    d.parts = sorted_parts(g, sorted_units(g.D));
+    a.joint = sorted_joint({g});
+    d.parts = sorted_parts(g, sorted_units(g.D), a.joint != 0);
     a.counter = (int *)ctx->sscr.p;
     a.ovf = (uint32_t *)((char *)ctx->sscr.p + 256);
     a.nfix = (const unsigned long long *)ctx->nfix.p;
@@ -1813,6 +1814,9 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
     std::vector<SortedItem> items;
     std::vector<int2> rmap, bmap;
     size_t so_ovf = 0;
+    std::vector<SysGeom> gs((size_t)n_sys);
+    for (int s = 0; s < n_sys; s++) gs[s] = sys[s].g;
+    const bool joint = srt && sorted_joint(gs);
     if (srt) {
         sos.resize((size_t)n_sys);
         int64_t units = 0;
@@ -1831,7 +1835,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
             q.list_ld = sorted_list_ld(L.g);
             q.row_first = 0;
             q.pad = sorted_pad(L.g.D);
-            q.parts = sorted_parts(L.g, units);
+            q.parts = sorted_parts(L.g, units, joint);
             sorted_items(s, L.g.D, 0, L.g.D, q.parts, items);
             for (int r = 0; r < L.g.D; r++) rmap.push_back(make_int2(s, r));
             for (int b = 0; b < sorted_blocks(L.g.D); b++) bmap.push_back(make_int2(s, b));
@@ -1848,8 +1852,6 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
         tiles.insert(tiles.end(), t.begin(), t.end());
         tsys.insert(tsys.end(), t.size(), s);
     }
-    std::vector<SysGeom> gs((size_t)n_sys);
-    for (int s = 0; s < n_sys; s++) gs[s] = sys[s].g;
     if (onehot) CK(ctx->ohbatch.ensure(pairs_onehot_batch_bytes(gs)));
     // preprocessing of all systems in one launch per input precision: CTA
     // k handles DOF map[k].y of system map[k].x
@@ -1905,6 +1907,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
     key.push_back(onehot ? (int64_t)(uintptr_t)ctx->ohbatch.p : -1);
     key.push_back(srt ? (int64_t)(uintptr_t)ctx->sscr.p : -1);
     key.push_back(tree);
+    key.push_back(joint);
     for (int k = 0; k < 6; k++) key.push_back(bins[k]);
     for (int s = 0; s < n_sys; s++) {
         const pg_bat_view &v = trajs[s];
@@ -1995,6 +1998,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
         else if (e == cudaSuccess && srt) {
             SortedArgs a{};
             a.many = (const SortedSys *)(meta + mo_so);
+            a.joint = joint;
             a.items = (const SortedItem *)(meta + mo_si);
             a.n_items = (int)items.size();
             a.counter = (int *)ctx->sscr.p;

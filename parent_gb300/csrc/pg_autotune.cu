@@ -309,7 +309,12 @@ int hist_layout(const SysGeom &g) {
 // DOFs x 60k x 90 bins 24.1 -> 10.5 ms; 603 DOFs x 20k x 51 bins 1.37 -> 1.11,
 // 444 DOFs x 5k 0.36 -> 0.38; 294 DOFs x 5k x 64 bins 0.39 -> 0.29, 174 DOFs
 // x 20k 0.24 -> 0.29; 294 DOFs x 5k x 160 bins 1.60 -> 1.21, 174 DOFs 0.57 ->
-// 0.74. A batch counts as one system of all its slots and pairs.
+// 0.74. To 35 bins the other kernel has 32-bit counters and no folds: 2,994
+// DOFs x 100k x 30 bins 76.8 -> 71.8, x 5k 8.2 -> 6.2, 1,494 DOFs x 100k 19.2
+// -> 18.9, x 5k 1.96 -> 1.71, 894 DOFs x 500k 32.9 -> 35.2; with joint counters
+// 2,994 DOFs x 100k x 16 bins 78.4 -> 55.3, 894 DOFs x 500k x 20 bins 34.4 ->
+// 29.5, 603 DOFs x 50k x 14 bins 1.67 -> 1.54. A batch counts as one system of
+// all its slots and pairs.
 // PG_HIST_SORTED=0|1 forces it off or on; PG_HIST_SLOTS and PG_HIST_STREAM
 // choose among the other kernels.
 bool sorted_layout(const std::vector<SysGeom> &gs) {
@@ -322,7 +327,18 @@ bool sorted_layout(const std::vector<SysGeom> &gs) {
         slots += (double)sorted_units(g.D) * 128.0 * g.F;
         pairs += 0.5 * g.D * (g.D - 1.0) * g.F;
     }
-    return bm > 35 && slots < pairs * (bm <= 50 ? 1.18 : (bm <= 57 ? 1.25 : 1.7));
+    if (bm <= 35) return slots < pairs * (sorted_joint(gs) ? 1.22 : 1.09);
+    return slots < pairs * (bm <= 50 ? 1.18 : (bm <= 57 ? 1.25 : 1.7));
+}
+
+// Seconds of the sorted-list kernel's pair phase, fitted to the times above
+// and those at 10 to 35 bins x 5k to 100k frames (within 8 %): counted slots
+// at the kernel's rate, and a read-out per row and block that grows with the
+// counters.
+static double sorted_seconds(const SysGeom &g, bool joint) {
+    const double units = (double)sorted_units(g.D), slots = units * 128.0, b = bmax_of(g);
+    return joint ? slots * g.F / 9.75e12 + units * 3.5e-11 * b * b * b
+                 : slots * g.F / 6.38e12 + units * (1.2e-8 + 8e-11 * b * b);
 }
 
 int layout_codes(int layout, int bmax) { return layout != HIST16 && !pairs_hist32_wide(bmax) ? 1 : 0; }
@@ -340,6 +356,7 @@ double predict_pair_seconds(const SysGeom &g, int form) {
         const double waves = ceil((double)pairs_onehot_tiles(h) / std::max(1, sms / 2));
         return c.call + waves * (c.t0 + c.t1 * g.F);
     }
+    if (sorted_layout({g})) return 5e-5 + sorted_seconds(g, sorted_joint({g}));
     const int layout = hist_layout(g);
     const SysGeom h = as_hist(g, layout);
     const TileCost c = cost_of(h, 1 + (layout == HIST16 ? 0 : layout));
@@ -383,11 +400,12 @@ int autotune_batch_form(const std::vector<SysGeom> &gs) {
             if (!fallback_onehot(g)) return PG_FORM_HIST;
         return PG_FORM_ONEHOT;
     }
+    const bool sorted = sorted_layout(gs), joint = sorted && sorted_joint(gs);
     for (const SysGeom &g : gs) {
         const int layout = hist_layout(g);
-        const TileCost ch = cost_of(as_hist(g, layout), 1 + (layout == HIST16 ? 0 : layout));
+        const TileCost ch = sorted ? TileCost{} : cost_of(as_hist(g, layout), 1 + (layout == HIST16 ? 0 : layout));
         const TileCost co = cost_of(as_onehot(g), 0);
-        if (!ch.ok || !co.ok) {
+        if ((!sorted && !ch.ok) || !co.ok) {
             for (const SysGeom &x : gs)
                 if (!fallback_onehot(x)) return PG_FORM_HIST;
             return PG_FORM_ONEHOT;
@@ -402,7 +420,7 @@ int autotune_batch_form(const std::vector<SysGeom> &gs) {
         }
         // one launch for the whole batch (its set-up runs once, outside the
         // replayed graph)
-        th += (double)tiles * (ch.t0 + ch.t1 * g.F) / sms;
+        th += sorted ? sorted_seconds(g, joint) : (double)tiles * (ch.t0 + ch.t1 * g.F) / sms;
         to += (double)pairs_onehot_tiles(as_onehot(g)) * (co.t0 + co.t1 * g.F) / std::max(1, sms / 2);
     }
     return to < th ? PG_FORM_ONEHOT : PG_FORM_HIST;

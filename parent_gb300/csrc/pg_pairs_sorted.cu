@@ -19,8 +19,8 @@
 // columns 16 sub .. 16 sub + 15 of frame fr.
 //
 // Counters. 16-bit halves: columns 2h and 2h + 1 of a 16-column group share a
-// word. A team's table has two planes (h >> 2) of one 32-word row per bin, and
-// the word of (sub, h) is sub * 4 + (h & 3): at every step the four frames of
+// word. The tables lie in two planes (h >> 2) at a fixed distance, a 32-word
+// row per bin in each, and the word of (sub, h) is sub * 4 + (h & 3): at every step the four frames of
 // a load take four different h of one plane (their order rotated by fr), so
 // the 32 lanes of a reduction lie in 32 banks. A half cannot pass the frames counted since
 // the last read-out, so pieces of at most kPiece frames never overflow;
@@ -31,6 +31,17 @@
 // kernels' bit for bit) and the occupied bins, kept in registers over the
 // segments of an item and added to the MI matrix's storage, which the
 // finishing kernel turns into S2D and MI.
+//
+// Joint counters (JOINT, up to 30 bins). Two neighbouring columns share one
+// counter per cell of their joint histogram, and one reduction counts both:
+// the rows hold the cell's code of every column pair (joint_code: the word in
+// the low bits, which half of it in the top bit), and the pair's marginals are
+// summed from the table at the read-out. A word holds the cells (b1, 2j) and
+// (b1, 2j + 1) as lo = n_even + n_odd and hi = -n_odd mod 65536 (the value
+// added comes from one byte permute of the code's top bit), so sums of words
+// are such pairs too. The read-out costs B^2 / 2 words a column pair, so it
+// takes long segments: sorted_joint. 2,994 DOFs x 100k frames, 16 bins: 73.2
+// ms with a counter per column, 55.3 with joint ones.
 //
 // What bounds it: the shared-memory / L1 data pipe, 91 % busy (894 DOFs x 100k
 // frames, 50 bins), two thirds of it the reductions: one cycle per 32 updates,
@@ -45,6 +56,7 @@
 // reductions one more cycle (160 KB of counters: 8.3e12 reductions of this
 // loop per second against 10.4e12 below 128 KB).
 #include <stdint.h>
+#include <stdlib.h>
 
 #include <algorithm>
 #include <vector>
@@ -64,10 +76,11 @@ using namespace dev;
 constexpr int kWarps = 16, kThreads = kWarps * 32;
 constexpr int kLoads = 8, kBatch = 4 * kLoads;  // row loads in flight per warp, and their frames
 constexpr int kBlk = 128;                 // columns of a block: bytes of a row
-constexpr int kRowBytes = 256;            // a team's counters of one bin
-constexpr int kTableMax = 120 * 1024;     // counter bytes of a CTA
+constexpr int kPlane = 60 * 1024;         // bytes of a plane: all teams' rows of 128 bytes
+constexpr int kPlaneWords = kPlane / 4;
 constexpr int kPiece = 64512;             // frames between read-outs: a half holds 65,535
 constexpr int kMaxTeams = 8;
+constexpr int kJointMax = 30;             // 451 rows of joint counters, 115 KB
 
 // ------------------------------------------------------------ preparation
 
@@ -155,9 +168,14 @@ __global__ void __launch_bounds__(kSortThreads) sort_frames_kernel(const __grid_
 
 // DOF-major bins -> blocks of 128 columns, frame-major: 256 frames of one
 // block per CTA through shared memory; a thread writes 32 columns (a whole
-// sector) of one frame. Columns outside the system and row F get the dummy
-// bin a.dummy.
+// sector) of one frame. Columns outside the system and row F count in the
+// tables' last row.
 constexpr int kTrFrames = 256, kTrPitch = kTrFrames + 4;
+
+// the cell of bins (b1, b2): row b1 * half + b2 / 2, the top bit for odd b2
+__device__ __forceinline__ uint32_t joint_code(uint32_t b1, uint32_t b2, int half) {
+    return b1 * (uint32_t)half + (b2 >> 1) | (b2 & 1u) << 15;
+}
 
 __global__ void __launch_bounds__(256) transpose_bins_kernel(const __grid_constant__ SortedArgs a, const int2 *map) {
     __shared__ uint8_t tile[kBlk * kTrPitch];
@@ -166,10 +184,12 @@ __global__ void __launch_bounds__(256) transpose_bins_kernel(const __grid_consta
     const int F = d.geo.F, f0 = blockIdx.x * kTrFrames;
     if (f0 > F) return;
     const int c0 = m.y * kBlk - d.pad;
-    const uint32_t dummy4 = 0x01010101u * (uint32_t)a.dummy;
+    // JOINT: a column outside the system has bin 0 (its partner's bins count)
+    const uint32_t dummy4 = a.joint ? 0x00010001u * (uint32_t)(a.rows - 1) : 0x01010101u * (uint32_t)a.bmax;
+    const uint32_t none = a.joint ? 0u : dummy4;
     for (int k = threadIdx.x; k < kBlk * (kTrFrames / 16); k += 256) {
         const int r = k / (kTrFrames / 16), q = (k % (kTrFrames / 16)) * 16, c = c0 + r;
-        uint4 v = make_uint4(dummy4, dummy4, dummy4, dummy4);
+        uint4 v = make_uint4(none, none, none, none);
         if (c >= 0 && f0 + q < F) v = __ldg((const uint4 *)(d.bins + (int64_t)c * d.geo.ldb + f0 + q));
         uint32_t *t = (uint32_t *)(tile + r * kTrPitch + q);
         t[0] = v.x;
@@ -185,12 +205,11 @@ __global__ void __launch_bounds__(256) transpose_bins_kernel(const __grid_consta
         uint32_t w[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) {
-            if (f0 + f == F) {
-                w[j] = dummy4;
-            } else {
-                const uint8_t *t = tile + (q + 4 * j) * kTrPitch + f;
-                w[j] = t[0] | (uint32_t)t[kTrPitch] << 8 | (uint32_t)t[2 * kTrPitch] << 16 | (uint32_t)t[3 * kTrPitch] << 24;
-            }
+            const uint8_t *t = tile + (q + 4 * j) * kTrPitch + f;
+            const uint32_t b0 = t[0], b1 = t[kTrPitch], b2 = t[2 * kTrPitch], b3 = t[3 * kTrPitch];
+            if (f0 + f == F) w[j] = dummy4;
+            else if (a.joint) w[j] = joint_code(b0, b1, a.half) | joint_code(b2, b3, a.half) << 16;
+            else w[j] = b0 | b1 << 8 | b2 << 16 | b3 << 24;
         }
         uint4 *o = (uint4 *)(out + (int64_t)f * kBlk + q);
         o[0] = make_uint4(w[0], w[1], w[2], w[3]);
@@ -220,18 +239,34 @@ __device__ __forceinline__ void team_barrier(int team, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(threads) : "memory");
 }
 
+// *(addr + OFF) += v
+template <int OFF>
+__device__ __forceinline__ void red_at(uint32_t addr, uint32_t v) {
+    asm volatile("red.shared.add.u32 [%0+%2], %1;" ::"r"(addr), "r"(v), "n"(OFF));
+}
+
 // Counts the 16 columns that a lane holds of its frame.
-__device__ __forceinline__ void count_rows(const uint4 &x, bool swap, const uint32_t (&wgt)[2][2],
-                                           const uint32_t (&base)[4][2]) {
-    const uint32_t c[4] = {swap ? x.y : x.x, swap ? x.x : x.y, swap ? x.w : x.z, swap ? x.z : x.w};
+template <bool JOINT, int OFF>
+__device__ __forceinline__ void count_word(uint32_t c, const uint32_t (&wgt)[2][2], const uint32_t (&base)[2]) {
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-            red_add_nc(__dp4a(c[k], wgt[e][0], base[k][e]), 1u);
-            red_add_nc(__dp4a(c[k], wgt[e][1], base[k][e]), 65536u);
+    for (int e = 0; e < 2; e++) {
+        if (JOINT) {
+            uint32_t v;  // 0x00000001, or 0xffff0001 where the half-word's top bit is set
+            asm("prmt.b32 %0, %1, %2, %3;" : "=r"(v) : "r"(c), "r"(1u), "r"(wgt[e][1]));
+            red_at<OFF>(__dp2a_lo(c & 0x7fff7fffu, wgt[e][0], base[e]), v);
+        } else {
+            red_at<OFF>(__dp4a(c, wgt[e][0], base[e]), 1u);
+            red_at<OFF>(__dp4a(c, wgt[e][1], base[e]), 65536u);
         }
     }
+}
+template <bool JOINT>
+__device__ __forceinline__ void count_rows(const uint4 &x, bool swap, const uint32_t (&wgt)[2][2],
+                                           const uint32_t (&base)[2][2]) {
+    count_word<JOINT, 0>(swap ? x.y : x.x, wgt, base[0]);
+    count_word<JOINT, 0>(swap ? x.x : x.y, wgt, base[1]);
+    count_word<JOINT, kPlane>(swap ? x.w : x.z, wgt, base[0]);
+    count_word<JOINT, kPlane>(swap ? x.z : x.w, wgt, base[1]);
 }
 
 // One warp's place in the lists: 32 entries from `base` of segment a (n of
@@ -240,7 +275,8 @@ struct Place {
     int a, base, n;
 };
 
-template <bool BIG>
+// JOINT: a counter is a cell of two columns' joint histogram (see the top).
+template <bool BIG, bool JOINT>
 __global__ void __launch_bounds__(kThreads, 1) pairs_sorted_kernel(const __grid_constant__ SortedArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_item[kMaxTeams];
@@ -248,26 +284,28 @@ __global__ void __launch_bounds__(kThreads, 1) pairs_sorted_kernel(const __grid_
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wpt = kWarps / a.teams, team = warp / wpt, tw = warp % wpt, tthreads = wpt * 32;
     const int ttid = tw * 32 + lane;
-    uint32_t *table = (uint32_t *)(smem + (size_t)team * a.rows * kRowBytes);
-    for (int k = ttid * 4; k < a.rows * 64; k += tthreads * 4) *(uint4 *)(table + k) = make_uint4(0u, 0u, 0u, 0u);
+    const int trows = a.rows + (JOINT ? a.half : 0);
+    uint32_t *table = (uint32_t *)smem + team * trows * 32;  // + q * kPlaneWords
+    uint32_t *colsum = table + a.rows * 32;  // JOINT: the second columns' sums
+    for (int k = ttid; k < trows * 32; k += tthreads) table[k] = table[kPlaneWords + k] = 0u;
     team_barrier(team, tthreads);
 
     const int fr = lane >> 3, sub = lane & 7;
     const bool swap = (fr & 2) != 0, odd = (fr & 1) != 0;
-    // half-word pair e of register k after the swap: its word in bin 0, and the
-    // byte weights that add 128 (a row) times its low / high bin byte
-    uint32_t base[4][2], wgt[2][2];
+    // half-word e of register k after the swap (k + 2: the other plane): its word in row 0, and the
+    // weights that add 128 (a row) times its low / high bin byte, or times the
+    // half-word's row; JOINT: wgt[e][1] is the byte selector of its value
+    uint32_t base[2][2], wgt[2][2];
 #pragma unroll
     for (int e = 0; e < 2; e++) {
         const int h = e ^ (int)odd;
 #pragma unroll
-        for (int k = 0; k < 4; k++)
-            base[k][e] = smem_u32(table) + (uint32_t)(((k >> 1) * a.rows) * 32 + sub * 4 + ((k & 1) ^ (int)swap) * 2 + h) * 4;
-        wgt[e][0] = 128u << (16 * h);
-        wgt[e][1] = wgt[e][0] << 8;
+        for (int k = 0; k < 2; k++) base[k][e] = smem_u32(table) + (uint32_t)(sub * 4 + (k ^ (int)swap) * 2 + h) * 4;
+        wgt[e][0] = JOINT ? 128u << (8 * h) : 128u << (16 * h);
+        wgt[e][1] = JOINT ? (h ? 0xBB54u : 0x9954u) : wgt[e][0] << 8;
     }
     const uint64_t pol = row_policy();
-    uint32_t *ovf = BIG ? a.ovf + ((size_t)blockIdx.x * a.teams + team) * (size_t)a.rows * 128 : nullptr;
+    uint32_t *ovf = BIG ? a.ovf + ((size_t)blockIdx.x * a.teams + team) * (size_t)(a.bmax + 1) * 128 : nullptr;
 
     for (;;) {
         if (ttid == 0) s_item[team] = atomicAdd(a.counter, 1);
@@ -339,13 +377,13 @@ __global__ void __launch_bounds__(kThreads, 1) pairs_sorted_kernel(const __grid_
                     if (p0.n == kBatch && p1.n == kBatch) {  // whole batches, without a test per load
 #pragma unroll
                         for (int g = 0; g < kLoads; g++) {
-                            count_rows(v[g], swap, wgt, base);
+                            count_rows<JOINT>(v[g], swap, wgt, base);
                             v[g] = ldg_row(mat + (int64_t)__shfl_sync(0xffffffffu, f1, 4 * g + fr) * kBlk, pol);
                         }
                     } else {
 #pragma unroll
                         for (int g = 0; g < kLoads; g++) {
-                            if (4 * g < p0.n) count_rows(v[g], swap, wgt, base);
+                            if (4 * g < p0.n) count_rows<JOINT>(v[g], swap, wgt, base);
                             if (4 * g < p1.n) v[g] = ldg_row(mat + (int64_t)__shfl_sync(0xffffffffu, f1, 4 * g + fr) * kBlk, pol);
                         }
                     }
@@ -354,52 +392,116 @@ __global__ void __launch_bounds__(kThreads, 1) pairs_sorted_kernel(const __grid_
                     f1 = f2;
                 }
                 team_barrier(team, tthreads);
-                if (!BIG || p_end >= s_end) break;
-                // the piece's counts to the team's 32-bit sums
-                for (int b = tw; b < bblk; b += wpt) {
-#pragma unroll
-                    for (int q = 0; q < 2; q++) {
-                        const int w = (q * a.rows + b) * 32 + lane;
-                        const uint32_t x = table[w];
-                        if (x) {
-                            table[w] = 0u;
-                            ovf[2 * w] += x & 0xffffu;
-                            ovf[2 * w + 1] += x >> 16;
+                // read-out, zeroing the counters: into the sums of row bin s, or
+                // after all but its last piece into the team's 32-bit counts
+                const bool last = !BIG || p_end >= s_end;
+                auto take = [&](int b, int q, int h, uint32_t n) {
+                    if (BIG) {
+                        uint32_t *o = ovf + ((b * 2 + q) * 2 + h) * 32 + lane;
+                        if (!last) {
+                            if (n) atomicAdd(o, n);  // this lane's own word: no wait for it
+                            return;
+                        }
+                        if (spilled) {
+                            n += __ldcg(o);
+                            __stcg(o, 0u);
                         }
                     }
+                    if (n > 1u) snl[q][h] += __ldg(a.nfix + n);  // n ln n is 0 below 2
+                    occ[q] += n ? 1u << (16 * h) : 0u;           // at most 218 x 218 a half
+                };
+                if constexpr (JOINT) {
+                    // first columns: their bins' rows summed; the words go on to the
+                    // second columns' sums, two bins to a word
+                    for (int b = tw; b < bblk; b += wpt) {
+#pragma unroll
+                        for (int q = 0; q < 2; q++) {
+                            uint32_t *r = table + q * kPlaneWords + b * a.half * 32 + lane;
+                            const uint32_t cs = smem_u32(colsum + q * kPlaneWords + lane);
+                            uint32_t n = 0u;
+                            for (int j0 = 0; j0 < a.half; j0 += 8) {
+                                uint32_t x[8];
+#pragma unroll
+                                for (int j = 0; j < 8; j++) x[j] = j0 + j < a.half ? r[(j0 + j) * 32] : 0u;
+                                const uint32_t any = x[0] | x[1] | x[2] | x[3] | x[4] | x[5] | x[6] | x[7];
+                                if (!__any_sync(0xffffffffu, any)) continue;
+#pragma unroll
+                                for (int j = 0; j < 8; j++) {
+                                    if (j0 + j < a.half) {
+                                        r[(j0 + j) * 32] = 0u;
+                                        red_add_nc(cs + (j0 + j) * 128, x[j]);
+                                        n += x[j] & 0xffffu;
+                                    }
+                                }
+                            }
+                            take(b, q, 0, n);
+                        }
+                    }
+                    team_barrier(team, tthreads);
+                    for (int j = tw; j < a.half; j += wpt) {
+#pragma unroll
+                        for (int q = 0; q < 2; q++) {
+                            uint32_t *c = colsum + q * kPlaneWords + j * 32 + lane;
+                            const uint32_t x = *c, no = (0u - (x >> 16)) & 0xffffu;
+                            *c = 0u;
+                            take(2 * j, q, 1, (x & 0xffffu) - no);
+                            take(2 * j + 1, q, 1, no);
+                        }
+                    }
+                } else {
+                    // two rows at a time: words that no column of the warp counted in
+                    // cost a load and a vote
+                    for (int b = tw; b < bblk; b += 2 * wpt) {
+                        uint32_t x[4];
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const int r = b + (j >> 1) * wpt;
+                            x[j] = r < bblk ? table[(j & 1) * kPlaneWords + r * 32 + lane] : 0u;
+                        }
+                        if (!__any_sync(0xffffffffu, x[0] | x[1] | x[2] | x[3]) && !(BIG && spilled)) continue;
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const int r = b + (j >> 1) * wpt;
+                            if (r < bblk) table[(j & 1) * kPlaneWords + r * 32 + lane] = 0u;
+                        }
+                        if (BIG && !last) {
+#pragma unroll
+                            for (int j = 0; j < 4; j++) {
+                                take(b + (j >> 1) * wpt, j & 1, 0, x[j] & 0xffffu);
+                                take(b + (j >> 1) * wpt, j & 1, 1, x[j] >> 16);
+                            }
+                            continue;
+                        }
+                        uint32_t n[8];
+#pragma unroll
+                        for (int j = 0; j < 8; j++) n[j] = j & 1 ? x[j >> 1] >> 16 : x[j >> 1] & 0xffffu;
+                        if (BIG && spilled) {
+#pragma unroll
+                            for (int j = 0; j < 8; j++) {
+                                const int r = b + (j >> 2) * wpt;
+                                uint32_t *o = ovf + ((r * 2 + ((j >> 1) & 1)) * 2 + (j & 1)) * 32 + lane;
+                                if (r < bblk) {
+                                    n[j] += __ldcg(o);
+                                    __stcg(o, 0u);
+                                }
+                            }
+                        }
+                        unsigned long long val[8];  // the table reads of all eight counts together
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            val[j] = 0ull;
+                            if (n[j] > 1u) val[j] = __ldg(a.nfix + n[j]);
+                            occ[(j >> 1) & 1] += n[j] ? 1u << (16 * (j & 1)) : 0u;
+                        }
+#pragma unroll
+                        for (int j = 0; j < 8; j++) snl[(j >> 1) & 1][j & 1] += val[j];
+                    }
+                    team_barrier(team, tthreads);
                 }
+                if (last) break;
                 spilled = true;
                 p_end = min(s_end, p_end + kPiece);
-                team_barrier(team, tthreads);
             }
-            // read-out of row bin s, zeroing the counters: a word that no column
-            // of the warp counted in costs one load and a vote
-            for (int b = tw; b < bblk; b += 2 * wpt) {
-                uint32_t x[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int r = b + (j >> 1) * wpt;
-                    x[j] = r < bblk ? table[((j & 1) * a.rows + r) * 32 + lane] : 0u;
-                }
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int q = j & 1, w = (q * a.rows + b + (j >> 1) * wpt) * 32 + lane;
-                    uint32_t n0 = x[j] & 0xffffu, n1 = x[j] >> 16;
-                    if (BIG && spilled && b + (j >> 1) * wpt < bblk) {
-                        n0 += ovf[2 * w];
-                        n1 += ovf[2 * w + 1];
-                        ovf[2 * w] = 0u;
-                        ovf[2 * w + 1] = 0u;
-                    }
-                    if (__any_sync(0xffffffffu, n0 | n1)) {
-                        table[w] = 0u;
-                        if (n0 > 1u) snl[q][0] += __ldg(a.nfix + n0);  // n ln n is 0 below 2
-                        if (n1 > 1u) snl[q][1] += __ldg(a.nfix + n1);
-                        occ[q] += (n0 != 0u) + ((n1 != 0u) << 16);  // at most 218 x 218 a half
-                    }
-                }
-            }
-            team_barrier(team, tthreads);
         }
         unsigned long long *acc = (unsigned long long *)d.out.mi;
 #pragma unroll
@@ -475,11 +577,15 @@ int sm_count() {
     return n;
 }
 
-int table_rows(int bmax) { return bmax + 1; }
+// Rows of a team's plane: its counters, the last one for what does not count,
+// and the second columns' sums
+int joint_half(int bmax) { return (bmax + 1) / 2; }
+int table_rows(int bmax, bool joint) { return (joint ? bmax * joint_half(bmax) : bmax) + 1; }
+int team_rows(int bmax, bool joint) { return table_rows(bmax, joint) + (joint ? joint_half(bmax) : 0); }
 // teams of a CTA: as many tables as fit, a power of two
-int team_count(int bmax) {
+int team_count(int bmax, bool joint) {
     int t = kMaxTeams;
-    while (t > 1 && t * table_rows(bmax) * kRowBytes > kTableMax) t >>= 1;
+    while (t > 1 && t * team_rows(bmax, joint) * 128 > kPlane) t >>= 1;
     return t;
 }
 
@@ -492,13 +598,32 @@ size_t sorted_mat_bytes(const SysGeom &g) { return (size_t)sorted_blocks(g.D) * 
 // full is the first, which the fewest rows visit
 int sorted_pad(int D) { return sorted_blocks(D) * kBlk - D; }
 size_t sorted_ovf_bytes(const SysGeom &g) {
-    return g.F > kPiece ? (size_t)sm_count() * team_count(bmax2d(g)) * table_rows(bmax2d(g)) * 128 * sizeof(uint32_t) : 0;
+    const int bm = bmax2d(g);
+    const int teams = bm <= kJointMax ? kMaxTeams : team_count(bm, false);
+    return g.F > kPiece ? (size_t)sm_count() * teams * (bm + 1) * 128 * sizeof(uint32_t) : 0;
+}
+
+// Joint counters: half the reductions (14 data-pipe cycles per load of 4 rows
+// against 22), but a read-out of B^2 / 2 words a column pair instead of 2 B.
+// F >= 5 B^3 from the times of both (2,994 DOFs): 10 bins x 5k frames 4.40 ms
+// plain and 3.85 joint, 14 x 5k 4.55 and 5.48, 16 x 20k 15.5 and 15.4, 20 x
+// 20k 15.8 and 19.3, 20 x 100k 73.7 and 59.0, 25 x 100k 74.5 and 72.0, 30 x
+// 100k 71.8 and 76.9. PG_SORTED_JOINT=0|1 forces it.
+bool sorted_joint(const std::vector<SysGeom> &gs) {
+    if (const char *e = getenv("PG_SORTED_JOINT")) return atoi(e) != 0 && bmax2d(gs[0]) <= kJointMax;
+    double f = 0.0, u = 0.0;
+    for (const SysGeom &g : gs) {
+        f += (double)sorted_units(g.D) * g.F;
+        u += (double)sorted_units(g.D);
+    }
+    const double b = bmax2d(gs[0]);
+    return b <= kJointMax && f >= 5.0 * b * b * b * u;
 }
 
 // Items per (row, block) unit: enough to give every team work, and about 24
 // rounds of items where that leaves an item 4,096 frames.
-int sorted_parts(const SysGeom &g, int64_t units) {
-    const int64_t slots = (int64_t)sm_count() * team_count(bmax2d(g));
+int sorted_parts(const SysGeom &g, int64_t units, bool joint) {
+    const int64_t slots = (int64_t)sm_count() * team_count(bmax2d(g), joint);
     units = std::max<int64_t>(units, 1);
     const int64_t fill = std::min<int64_t>((slots + units - 1) / units, bmax2d(g));
     const int64_t even = std::min<int64_t>((24 * slots + units - 1) / units, g.F / 4096);
@@ -526,9 +651,10 @@ void sorted_items(int s, int D, int row0, int row1, int parts, std::vector<Sorte
 
 static SortedArgs complete(const SortedArgs &in, int bmax) {
     SortedArgs a = in;
-    a.rows = table_rows(bmax);
-    a.teams = team_count(bmax);
-    a.dummy = bmax;
+    a.bmax = bmax;
+    a.half = joint_half(bmax);
+    a.rows = table_rows(bmax, a.joint != 0);
+    a.teams = team_count(bmax, a.joint != 0);
     return a;
 }
 
@@ -553,8 +679,9 @@ cudaError_t launch_pairs_sorted(const SortedArgs &in, int bmax, bool big, cudaSt
     if (a.n_items <= 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(a.counter, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
-    const size_t smem = (size_t)a.teams * a.rows * kRowBytes;
-    auto kern = big ? pairs_sorted_kernel<true> : pairs_sorted_kernel<false>;
+    const size_t smem = kPlane + (size_t)a.teams * team_rows(bmax, a.joint != 0) * 128;
+    auto kern = a.joint ? (big ? pairs_sorted_kernel<true, true> : pairs_sorted_kernel<false, true>)
+                        : (big ? pairs_sorted_kernel<true, false> : pairs_sorted_kernel<false, false>);
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int grid = std::min(sm_count(), (a.n_items + a.teams - 1) / a.teams);

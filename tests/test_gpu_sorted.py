@@ -61,22 +61,36 @@ def test_sorted_equals_tiled_and_oracle(eng, monkeypatch, atoms, frames, b2, pre
     assert np.max(np.abs(a - ref)) <= 1e-9
 
 
+# 1 to 8 warps per table and one table per CTA; odd and mixed bin counts, a
+# column pair over a block's first column and over a change of type
+JOINT = [(3, 5, (30, 30, 30), 0), (44, 31, (7, 8, 9), 1), (45, 997, (1, 2, 3), 0), (88, 4097, (10, 10, 10), 0),
+         (30, 4096, (15, 14, 16), 1), (60, 2500, (20, 21, 19), 0), (24, 20001, (30, 29, 17), 0)]
+
+
+@pytest.mark.parametrize("atoms,frames,b2,prec", JOINT)
+def test_joint_counters_equal_tiled_and_oracle(eng, monkeypatch, atoms, frames, b2, prec):
+    monkeypatch.setenv("PG_SORTED_JOINT", "1")
+    test_sorted_equals_tiled_and_oracle(eng, monkeypatch, atoms, frames, b2, prec)
+
+
+@pytest.mark.parametrize("bins,joint", [(50, "0"), (20, "1")])
 @pytest.mark.parametrize("frames", [64512, 64513, 140000])
-def test_sorted_counts_above_16_bits(eng, monkeypatch, frames):
+def test_sorted_counts_above_16_bits(eng, monkeypatch, frames, bins, joint):
     """Columns with one value in most frames: segments and counts around and
     past what a 16-bit half holds (pieces of 64,512 frames)."""
+    monkeypatch.setenv("PG_SORTED_JOINT", joint)
     t = pg.synth_host(9, frames, double_prec=0, seed=5)
     for k, c in enumerate((t.bonds, t.angles, t.dihedrals)):
         c[:, : frames - 7 - k] = c[:, :1]
-    (a, ea, _), (b, eb, _) = _both(eng, monkeypatch, t, (50,) * 6)
+    (a, ea, _), (b, eb, _) = _both(eng, monkeypatch, t, (bins,) * 6)
     assert np.array_equal(a, b) and np.array_equal(ea, eb)
 
 
-def test_sorted_batch_equals_single_calls(eng, monkeypatch):
+@pytest.mark.parametrize("bins", [(50, 50, 50, 50, 44, 39), (10, 10, 10, 9, 10, 8)])
+def test_sorted_batch_equals_single_calls(eng, monkeypatch, bins):
     """One launch over systems of several sizes, replayed, against a call per
-    system (the batch's items are split differently)."""
+    system (the batch's items are split differently); 10 bins: joint counters."""
     monkeypatch.setenv("PG_HIST_SORTED", "1")
-    bins = (50, 50, 50, 50, 44, 39)
     trajs = [pg.synth_host(a, f, double_prec=p, seed=k) for k, (a, f, p) in
              enumerate([(50, 5000, 0), (4, 64600, 1), (90, 333, 1), (45, 9000, 0)])]
     single = []
