@@ -299,46 +299,59 @@ int hist_layout(const SysGeom &g) {
     return pairs_hist32_supported(bm) ? HIST32_STREAM : HIST16;
 }
 
-// The sorted-list kernel, from pair-phase times against the kernel that
-// hist_layout picks (same system, one call after the other). It counts whole
-// blocks of 128 columns, of which a small system leaves many empty; the line
-// is drawn on the counted slots per pair (2,994 DOFs: 1.04, 894: 1.14, 603:
-// 1.21, 444: 1.29, 294: 1.57, 174: 1.85). 36-50 bins: 2,994 DOFs x 100k frames
-// 90.5 -> 73.8 ms at 50 bins, 894 DOFs 8.2 -> 7.9, 603 DOFs 3.82 -> 4.00.
-// Above 50 bins the other kernel holds 4 pairs per CTA (to 100), then 1: 1,194
-// DOFs x 60k x 90 bins 24.1 -> 10.5 ms; 603 DOFs x 20k x 51 bins 1.37 -> 1.11,
-// 444 DOFs x 5k 0.36 -> 0.38; 294 DOFs x 5k x 64 bins 0.39 -> 0.29, 174 DOFs
-// x 20k 0.24 -> 0.29; 294 DOFs x 5k x 160 bins 1.60 -> 1.21, 174 DOFs 0.57 ->
-// 0.74. To 35 bins the other kernel has 32-bit counters and no folds: 2,994
-// DOFs x 100k x 30 bins 76.8 -> 71.8, x 5k 8.2 -> 6.2, 1,494 DOFs x 100k 19.2
-// -> 18.9, x 5k 1.96 -> 1.71, 894 DOFs x 500k 32.9 -> 35.2; with joint counters
-// 2,994 DOFs x 100k x 16 bins 78.4 -> 55.3, 894 DOFs x 500k x 20 bins 34.4 ->
-// 29.5, 603 DOFs x 50k x 14 bins 1.67 -> 1.54. A batch counts as one system of
-// all its slots and pairs.
-// PG_HIST_SORTED=0|1 forces it off or on; PG_HIST_SLOTS and PG_HIST_STREAM
-// choose among the other kernels.
+// Pair-phase seconds of the histogram kernels, fitted to both measured on one
+// system after the other (66 to 2,994 DOFs x 1k to 100k frames x 10 to 200
+// bins; every time within 35 %, 5 to 8 % rms): the counting, per counted slot
+// or pair and frame; the read-out, per row and block or per pair, which grows
+// with the counters; the lists and the transposition, per value; the launches.
+// Sorted lists count whole blocks of 128 columns (2,994 DOFs: 1.04 slots a
+// pair, 603: 1.21, 294: 1.57) and read their counters once per row bin. Tiles
+// count pairs exactly, with 32-bit counters to 35 bins, 16-bit to 50, then 16
+// pairs a CTA, 4 from 58 bins and 1 above 100. Some of both, in ms:
+//   2,994 DOFs x 100k: 10 bins 80.7 tiles, 68.8 lists, 51.5 joint; 20 bins 78.3,
+//     69.5, 60.1; 30 bins 76.7, 70.8, 77.6; 50 bins 90.5, 71.5; 64 bins 213, 75.0
+//   2,994 DOFs x 1k: 10 bins 4.12, 1.43, 2.02; 50 bins 8.09, 6.51
+//   894 DOFs x 100k: 30 bins 6.96, 7.26; 50 bins 8.21, 7.29; x 5k: 30 bins 0.72,
+//     0.64; 50 bins 1.06, 0.93
+//   603 DOFs x 20k: 20 bins 0.77, 0.85; 50 bins 1.03, 1.01; 51 bins 1.37, 1.02
+//   294 DOFs x 20k: 50 bins 0.28, 0.38; 64 bins 0.65, 0.41; 174 DOFs x 20k x 64
+//     bins 0.24 both
+static double tiled_seconds(const SysGeom &g) {
+    const double p = 0.5 * g.D * (g.D - 1.0), F = g.F, b = bmax_of(g), b2 = b * b;
+    if (b <= 35) return p * (1.71e-13 * F + 6.5e-10 + 3.4e-13 * b2);
+    if (b <= 50) return p * (1.96e-13 * F + 4.6e-10 + 4.6e-13 * b2);
+    if (b <= 57) return p * (2.54e-13 * F + 9.2e-13 * b2);
+    if (b <= 100) return p * (4.03e-13 * F + 5.2e-9 + 4.1e-13 * b2);
+    return p * (9.96e-13 * F + 2.15e-8 + 3.9e-13 * b2);
+}
+static double sorted_seconds(const SysGeom &g, bool joint) {
+    const double u = (double)sorted_units(g.D), F = g.F, b = bmax_of(g);
+    if (joint) return u * (128 * 9.8e-14 * F + 1.5e-8 + 2.35e-11 * b * b * b) + 1.2e-11 * g.D * F;
+    return u * (128 * (b < 118 ? 1.31e-13 : 1.62e-13) * F + 1e-8 + 6.4e-11 * b * b) + 9e-12 * g.D * F;
+}
+static constexpr double kTiledCall = 2e-5, kSortedCall = 8e-5;
+static double sum_sorted(const std::vector<SysGeom> &gs, bool joint) {
+    double s = kSortedCall;
+    for (const SysGeom &g : gs) s += sorted_seconds(g, joint);
+    return s;
+}
+
+// Joint counters (PG_SORTED_JOINT=0|1 forces the choice where they fit).
+bool sorted_joint(const std::vector<SysGeom> &gs) {
+    if (!sorted_joint_fits(bmax_of(gs[0]))) return false;
+    if (const char *e = getenv("PG_SORTED_JOINT")) return atoi(e) != 0;
+    return sum_sorted(gs, true) < sum_sorted(gs, false);
+}
+
+// A batch counts as the sum of its systems. PG_HIST_SORTED=0|1 forces the
+// choice; PG_HIST_SLOTS and PG_HIST_STREAM choose among the tiled kernels.
 bool sorted_layout(const std::vector<SysGeom> &gs) {
     if (const char *e = getenv("PG_HIST_SORTED")) return atoi(e) != 0;
     if (getenv("PG_HIST_SLOTS") || getenv("PG_HIST_STREAM")) return false;
-    double slots = 0.0, pairs = 0.0;
-    int bm = 0;
-    for (const SysGeom &g : gs) {
-        bm = std::max(bm, bmax_of(g));
-        slots += (double)sorted_units(g.D) * 128.0 * g.F;
-        pairs += 0.5 * g.D * (g.D - 1.0) * g.F;
-    }
-    if (bm <= 35) return slots < pairs * (sorted_joint(gs) ? 1.22 : 1.09);
-    return slots < pairs * (bm <= 50 ? 1.18 : (bm <= 57 ? 1.25 : 1.7));
-}
-
-// Seconds of the sorted-list kernel's pair phase, fitted to the times above
-// and those at 10 to 35 bins x 5k to 100k frames (within 8 %): counted slots
-// at the kernel's rate, and a read-out per row and block that grows with the
-// counters.
-static double sorted_seconds(const SysGeom &g, bool joint) {
-    const double units = (double)sorted_units(g.D), slots = units * 128.0, b = bmax_of(g);
-    return joint ? slots * g.F / 9.75e12 + units * 3.5e-11 * b * b * b
-                 : slots * g.F / 6.38e12 + units * (1.2e-8 + 8e-11 * b * b);
+    double tiled = kTiledCall;
+    for (const SysGeom &g : gs) tiled += tiled_seconds(g);
+    // 0.92: at no point of the measured grid slower than the tiles
+    return sum_sorted(gs, sorted_joint(gs)) < 0.92 * tiled;
 }
 
 int layout_codes(int layout, int bmax) { return layout != HIST16 && !pairs_hist32_wide(bmax) ? 1 : 0; }
@@ -356,7 +369,7 @@ double predict_pair_seconds(const SysGeom &g, int form) {
         const double waves = ceil((double)pairs_onehot_tiles(h) / std::max(1, sms / 2));
         return c.call + waves * (c.t0 + c.t1 * g.F);
     }
-    if (sorted_layout({g})) return 5e-5 + sorted_seconds(g, sorted_joint({g}));
+    if (sorted_layout({g})) return sum_sorted({g}, sorted_joint({g}));
     const int layout = hist_layout(g);
     const SysGeom h = as_hist(g, layout);
     const TileCost c = cost_of(h, 1 + (layout == HIST16 ? 0 : layout));

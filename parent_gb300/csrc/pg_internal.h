@@ -288,7 +288,8 @@ struct SortedArgs {
     int joint;             // sorted_joint
     int bmax, half, rows, teams;  // set by the launchers
 };
-bool sorted_joint(const std::vector<SysGeom> &gs);
+bool sorted_joint_fits(int bmax);
+bool sorted_joint(const std::vector<SysGeom> &gs);  // pg_autotune.cu
 int64_t sorted_list_ld(const SysGeom &g);
 int sorted_blocks(int D);
 size_t sorted_mat_bytes(const SysGeom &g);

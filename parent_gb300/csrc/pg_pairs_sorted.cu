@@ -39,8 +39,9 @@
 // summed from the table at the read-out. A word holds the cells (b1, 2j) and
 // (b1, 2j + 1) as lo = n_even + n_odd and hi = -n_odd mod 65536 (the value
 // added comes from one byte permute of the code's top bit), so sums of words
-// are such pairs too. The read-out costs B^2 / 2 words a column pair, so it
-// takes long segments: sorted_joint. 2,994 DOFs x 100k frames, 16 bins: 73.2
+// are such pairs too. Half the reductions (14 data-pipe cycles per load of 4
+// rows against 22), but a read-out of B^2 / 2 words a column pair instead of 2
+// B, so long segments only (sorted_joint). 2,994 DOFs x 100k frames, 16 bins: 73.2
 // ms with a counter per column, 55.3 with joint ones.
 //
 // What bounds it: the shared-memory / L1 data pipe, 91 % busy (894 DOFs x 100k
@@ -56,7 +57,6 @@
 // reductions one more cycle (160 KB of counters: 8.3e12 reductions of this
 // loop per second against 10.4e12 below 128 KB).
 #include <stdint.h>
-#include <stdlib.h>
 
 #include <algorithm>
 #include <vector>
@@ -603,22 +603,7 @@ size_t sorted_ovf_bytes(const SysGeom &g) {
     return g.F > kPiece ? (size_t)sm_count() * teams * (bm + 1) * 128 * sizeof(uint32_t) : 0;
 }
 
-// Joint counters: half the reductions (14 data-pipe cycles per load of 4 rows
-// against 22), but a read-out of B^2 / 2 words a column pair instead of 2 B.
-// F >= 5 B^3 from the times of both (2,994 DOFs): 10 bins x 5k frames 4.40 ms
-// plain and 3.85 joint, 14 x 5k 4.55 and 5.48, 16 x 20k 15.5 and 15.4, 20 x
-// 20k 15.8 and 19.3, 20 x 100k 73.7 and 59.0, 25 x 100k 74.5 and 72.0, 30 x
-// 100k 71.8 and 76.9. PG_SORTED_JOINT=0|1 forces it.
-bool sorted_joint(const std::vector<SysGeom> &gs) {
-    if (const char *e = getenv("PG_SORTED_JOINT")) return atoi(e) != 0 && bmax2d(gs[0]) <= kJointMax;
-    double f = 0.0, u = 0.0;
-    for (const SysGeom &g : gs) {
-        f += (double)sorted_units(g.D) * g.F;
-        u += (double)sorted_units(g.D);
-    }
-    const double b = bmax2d(gs[0]);
-    return b <= kJointMax && f >= 5.0 * b * b * b * u;
-}
+bool sorted_joint_fits(int bmax) { return bmax <= kJointMax; }
 
 // Items per (row, block) unit: enough to give every team work, and about 24
 // rounds of items where that leaves an item 4,096 frames.
