@@ -1055,6 +1055,16 @@ PG_API int pg_bat_from_cartesian(pg_ctx *ctx, const float *xyz, int xyz_on_devic
         atoms[i] = make_int4(r[0] - 1, r[1] - 1, r[2] - 1, r[3] - 1);
         parent[i] = r[5] == -1 ? -1 : r[5] - 1;
     }
+    // links of a dihedral: its ancestors that come before their child, whose
+    // phase angles it is taken from; a later parent is read raw
+    parent.resize(2 * (size_t)nd);
+    int links = 0;
+    for (int i = 0; i < nd; i++) {
+        const int p = parent[i];
+        parent[nd + i] = p >= 0 && p < i ? parent[nd + p] + 1 : 0;
+        links = std::max(links, parent[nd + i]);
+    }
+    const bool tmp_own = !double_prec || bat_phase_short(links);  // raw dihedrals outside the output
     CK(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     const int64_t F = n_frames, ld = (F + 31) / 32 * 32;
@@ -1063,16 +1073,16 @@ PG_API int pg_bat_from_cartesian(pg_ctx *ctx, const float *xyz, int xyz_on_devic
     const int64_t lds = (fc + 31) / 32 * 32;
     CK(ctx->bc_out.ensure((size_t)(3 * (int64_t)nd + 3) * ld * es));
     CK(ctx->bc_soa.ensure((size_t)3 * na * lds * sizeof(float)));
-    if (!double_prec) CK(ctx->bc_tmp.ensure((size_t)nd * lds * sizeof(double)));
+    if (tmp_own) CK(ctx->bc_tmp.ensure((size_t)nd * lds * sizeof(double)));
     // host coordinates the GPU can read go straight into the transpose (one
     // read over the host link), the others through a staging copy
     const bool stage = !xyz_on_device && !host_readable(xyz);
     if (stage) CK(ctx->bc_stage.ensure((size_t)fc * na * 3 * sizeof(float)));
-    CK(ctx->bc_tab.ensure((size_t)nd * (sizeof(int4) + sizeof(int))));
+    CK(ctx->bc_tab.ensure((size_t)nd * (sizeof(int4) + 2 * sizeof(int))));
     int4 *d_atoms = (int4 *)ctx->bc_tab.p;
     int *d_parent = (int *)(d_atoms + nd);
     CK(cudaMemcpyAsync(d_atoms, atoms.data(), sizeof(int4) * nd, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(d_parent, parent.data(), sizeof(int) * nd, cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(d_parent, parent.data(), sizeof(int) * 2 * nd, cudaMemcpyHostToDevice, st));
     char *o = (char *)ctx->bc_out.p;
     void *bonds = o, *angles = o + (size_t)(nd + 2) * ld * es, *dihs = o + (size_t)(2 * nd + 3) * ld * es;
     CK(cudaEventRecord(ctx->ev[0], st));
@@ -1084,11 +1094,11 @@ PG_API int pg_bat_from_cartesian(pg_ctx *ctx, const float *xyz, int xyz_on_devic
             src = (const float *)ctx->bc_stage.p;
         }
         CK(launch_cart_transpose(src, n, na, (float *)ctx->bc_soa.p, lds, st));
-        double *tmp = double_prec ? (double *)dihs + f0 : (double *)ctx->bc_tmp.p;
-        const int64_t ldt = double_prec ? ld : lds;
+        double *tmp = tmp_own ? (double *)ctx->bc_tmp.p : (double *)dihs + f0;
+        const int64_t ldt = tmp_own ? lds : ld;
         CK(launch_bat_convert((const float *)ctx->bc_soa.p, lds, n, nd, d_atoms, bonds, angles, ld, f0, double_prec,
                               tmp, ldt, st));
-        CK(launch_bat_phase(tmp, ldt, n, nd, d_parent, dihs, ld, f0, double_prec, st));
+        CK(launch_bat_phase(tmp, ldt, n, nd, d_parent, links, dihs, ld, f0, double_prec, st));
         ctx->launches += 3;
     }
     CK(cudaEventRecord(ctx->ev[1], st));

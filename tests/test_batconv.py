@@ -179,3 +179,39 @@ def test_gpu_conversion_from_device_coordinates():
         got = _cols(v)
     for g, w in zip(got, want):
         assert np.array_equal(g, w)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["branched", "eight links", "nine links", "lines"])
+def test_gpu_conversion_branches_match_oracle(kind):
+    """Dihedrals that do and do not take over their predecessor's vectors,
+    chains of parents at and past what the parallel phase kernel takes, atoms
+    on a line and on one another (the library's acos, NaN where the reference
+    divides 0 by 0)."""
+    rng = np.random.default_rng(11)
+    xyz, dih = _chain(40, 257, 5)
+    n = dih.shape[0]
+    if kind == "branched":
+        for i in range(n):
+            if i % 2:
+                dih[i, :4] = rng.choice(40, 4, replace=False) + 1
+    if kind.endswith("links"):
+        k = 9 if kind == "eight links" else 10
+        dih[:, 5] = [-1 if i % k == 0 else i for i in range(n)]  # the previous dihedral, 1-based
+    if kind == "lines":
+        xyz[3::7, 10] = 2 * xyz[3::7, 9] - xyz[3::7, 8]   # atoms 9, 10, 11 on a line
+        xyz[4::7, 20] = xyz[4::7, 21]                      # two atoms in one place
+    for prec in (1, 0):
+        with pg.Engine(0) as eng:
+            got = _cols(eng.bat_from_cartesian(xyz, dih, prec))
+        want = oracle.bat_from_xyz(xyz, dih)
+        for k, (g, w) in enumerate(zip(got, want)):
+            w = w if prec else w.astype(np.float32)
+            assert np.array_equal(np.isnan(g), np.isnan(w))
+            ok = ~np.isnan(w)
+            if k == 0:
+                assert np.array_equal(g[ok], w[ok])
+            elif prec:
+                assert _angle_close(g[ok], w[ok], 1e-12)
+            else:
+                assert _angle_close(g[ok].astype(np.float64), w[ok].astype(np.float64), 5e-7)  # one float32 place of 2 pi
