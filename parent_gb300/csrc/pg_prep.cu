@@ -71,6 +71,18 @@ __device__ __forceinline__ F2 split2(double v) {
     return {hi, __double2float_rn(__dsub_rn(v, (double)hi))};
 }
 
+// A DOF's binning constants (bounds in prep_body), and those of every DOF.
+struct Bins {
+    double mn, bs1, bs2;
+    F2 mn2;
+    float r1, r2, e1, e2;
+};
+struct Consts {
+    double modfit_bs, pi;
+    float rm, r2pi;  // FP32 reciprocals of modfit_bs and 2 pi
+    F2 tp2;          // 2 pi
+};
+
 // Extrema of a dihedral column after the shift: within one value of
 // q = int((x + modFit) / 2 pi) the shifted value is a non-decreasing function
 // of x (FP64 rounding is monotone), so the largest / smallest x of each q
@@ -186,7 +198,8 @@ constexpr int kTail = 256;  // bins per chunk of the per-DOF sums
 template <typename T>
 __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, const void *ca, const void *cd,
                                           int64_t ld, int prec, const DofArrays &dof, uint8_t *bins, int *err,
-                                          double modfit_bs, double pi, int g, int h1_copies) {
+                                          const Consts &c, int g, int h1_copies) {
+    const double modfit_bs = c.modfit_bs, pi = c.pi;
     extern __shared__ unsigned int sh[];
     const int type = dof_type(g, geo.nb, geo.na);
     const int local = g - (type == TB ? 0 : (type == TA ? geo.nb : geo.nb + geo.na));
@@ -208,8 +221,9 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
     unsigned int *h1 = hmod + kWarps * kModfitBins;
     unsigned int *h2 = h1 + h1_copies * B1;  // per-warp 1D histograms, or one shared copy for large B1
     const int w1 = h1_copies > 1 ? warp : 0;
-    __shared__ double s_shift, s_mn, s_mx;
-    __shared__ double red_mn[kWarps], red_mx[kWarps];
+    __shared__ double s_shift;
+    __shared__ Bins s_bins;
+    __shared__ F2 s_mf2;
 
     double modfit = 0.0;
     if (type == TD) {
@@ -218,7 +232,7 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
         int bad = 0;
         // x / modfit_bs: relative error of x32 * fl32(1/bs) <= 2^-23 (2^-22.4
         // with the FP32 rounding of an FP64 input)
-        const float rm = __double2float_rn(__drcp_rn(modfit_bs));
+        const float rm = c.rm;
         for_frames<kUnroll, kThreads>(colT, F, tid, [&](int, T xv) {
             const float x = (float)xv;
             const float q = __fmul_rn(x, rm);
@@ -261,6 +275,7 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
             }
             // modFit = 2 pi - (pos + 0.5) * binsize, PARENT.cpp:609
             s_shift = __dsub_rn(twopi, __dmul_rn(__dadd_rn((double)longestPos, 0.5), modfit_bs));
+            s_mf2 = split2(s_shift);
         }
         __syncthreads();
         modfit = s_shift;
@@ -269,8 +284,8 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
     // FP32 images of the shift constants; t = x + modFit and its quotient by
     // 2 pi are screened with |t32 - t| <= 2^-23 (|x| + |modFit|) <= 2e-6 and
     // |q - t / 2 pi| <= 8e-7 for x < 2 pi + 5e-9, modFit <= 2 pi
-    const F2 mf2 = split2(modfit), tp2 = split2(twopi);
-    const float r2pi = __double2float_rn(__drcp_rn(twopi));
+    const F2 mf2 = type == TD ? s_mf2 : F2{0.f, 0.f}, tp2 = c.tp2;
+    const float r2pi = c.r2pi;
     constexpr float kShiftEps = 4e-6f;
     // exact quotient q of the shift of value xv: screened on its FP32
     // rounding, else FP64
@@ -335,17 +350,17 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
                 if (va > lmax) lmax = va;
                 if (vb < lmin) lmin = vb;
             }
-            red_mx[0] = lmax;
-            red_mn[0] = lmin;
         }
     }
-    __syncthreads();
+    // the DOF's constants, by one thread: the FP64 pipe takes one warp
+    // instruction per 16 cycles and SM, so a constant that all 16 warps form
+    // costs 16 times as much as one that a warp forms and the others read
+    // (294 DOFs x 20,000 frames, whole call: 891 -> 856 us; 66 DOFs x 2,000:
+    // 248 -> 234 us)
     if (tid == 0) {
         double tmpMax = -1.0e100, tmpMin = 1.0e100;
-        for (int w = 0; w < 1; w++) {
-            if (red_mx[w] > tmpMax) tmpMax = red_mx[w];
-            if (red_mn[w] < tmpMin) tmpMin = red_mn[w];
-        }
+        if (lmax > tmpMax) tmpMax = lmax;
+        if (lmin < tmpMin) tmpMin = lmin;
         if (type == TB && ((tmpMin < 0.0) || (tmpMax < 0.0))) atomicAdd(&err[ERR_NEG_BOND], 1);
         tmpMin = __dsub_rn(tmpMin, 0.000000005);
         tmpMax = __dadd_rn(tmpMax, 0.000000005);
@@ -353,8 +368,24 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
         if (type == TA && tmpMax > pi) tmpMax = pi;
         if (type == TD && tmpMax > twopi) tmpMax = twopi;
         if (__dsub_rn(tmpMax, tmpMin) < 1.0e-4) tmpMax = __dadd_rn(tmpMax, 0.05);
-        s_mn = tmpMin;
-        s_mx = tmpMax;
+        Bins b;
+        b.mn = tmpMin;
+        b.bs1 = __ddiv_rn(__dsub_rn(tmpMax, tmpMin), (double)B1);
+        b.bs2 = __ddiv_rn(__dsub_rn(tmpMax, tmpMin), (double)B2);
+        // d = fl64(x' - mn) (x' the shifted value for dihedrals) is formed in
+        // FP32 from split constants, |d32 - d| <= 2^-20 E with
+        // E = |mn| + |mx| (+ 2|modFit| + 8 pi for dihedrals), a bound >= 4x
+        // the accumulated rounding (including an FP64 input's rounding to
+        // FP32, <= 2^-24 E); q_k = d32 * fl32(1 / bs_k) then has
+        // |q_k - q*| <= 2^-20 E / bs_k + 2^-22 q_k.
+        b.mn2 = split2(tmpMin);
+        b.r1 = __double2float_rn(__drcp_rn(b.bs1));
+        b.r2 = __double2float_rn(__drcp_rn(b.bs2));
+        double E = fabs(tmpMin) + fabs(tmpMax);
+        if (type == TD) E = E + 2.0 * fabs(modfit) + 4.0 * twopi;
+        b.e1 = __double2float_ru(E * 0x1p-20 / b.bs1);
+        b.e2 = __double2float_ru(E * 0x1p-20 / b.bs2);
+        s_bins = b;
         dof.mn[g] = tmpMin;
         dof.mx[g] = tmpMax;
         dof.shift[g] = modfit;
@@ -364,22 +395,11 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
     __syncthreads();
 
     // ---- binning (PARENT.cpp:654-656 1D; :800-803 and the other 2D fills)
-    const double mn = s_mn, mx = s_mx;
-    const double bs1 = __ddiv_rn(__dsub_rn(mx, mn), (double)B1);
-    const double bs2 = __ddiv_rn(__dsub_rn(mx, mn), (double)B2);
+    const double mn = s_bins.mn, bs1 = s_bins.bs1, bs2 = s_bins.bs2;
     int bad = 0;
     {
-        // d = fl64(x' - mn) (x' the shifted value for dihedrals) is formed in
-        // FP32 from split constants, |d32 - d| <= 2^-20 E with
-        // E = |mn| + |mx| (+ 2|modFit| + 8 pi for dihedrals), a bound >= 4x
-        // the accumulated rounding (including an FP64 input's rounding to
-        // FP32, <= 2^-24 E); q_k = d32 * fl32(1 / bs_k) then has
-        // |q_k - q*| <= 2^-20 E / bs_k + 2^-22 q_k.
-        const F2 mn2 = split2(mn);
-        const float r1 = __double2float_rn(__drcp_rn(bs1)), r2 = __double2float_rn(__drcp_rn(bs2));
-        double E = fabs(mn) + fabs(mx);
-        if (type == TD) E = E + 2.0 * fabs(modfit) + 4.0 * twopi;
-        const float e1 = __double2float_ru(E * 0x1p-20 / bs1), e2 = __double2float_ru(E * 0x1p-20 / bs2);
+        const F2 mn2 = s_bins.mn2;
+        const float r1 = s_bins.r1, r2 = s_bins.r2, e1 = s_bins.e1, e2 = s_bins.e2;
         // both bin indices of one value, counted in the 1D histograms; the 2D
         // bin is returned for the pair kernels' bin matrices
         auto bin_of = [&](T xin) -> int {
@@ -535,8 +555,8 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
 template <typename T>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) prep_kernel(SysGeom geo, const void *cb, const void *ca, const void *cd,
                                                         int64_t ld, int prec, DofArrays dof, uint8_t *bins, int *err,
-                                                        double modfit_bs, double pi, int g_first, int h1_copies) {
-    prep_body<T>(geo, cb, ca, cd, ld, prec, dof, bins, err, modfit_bs, pi, g_first + blockIdx.x, h1_copies);
+                                                        const __grid_constant__ Consts c, int g_first, int h1_copies) {
+    prep_body<T>(geo, cb, ca, cd, ld, prec, dof, bins, err, c, g_first + blockIdx.x, h1_copies);
 }
 
 // Many systems in one launch: CTA k preprocesses DOF map[k].y of system
@@ -544,11 +564,10 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) prep_kernel(SysGeom geo,
 template <typename T>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) prep_batch_kernel(const PrepDesc *__restrict__ sys,
                                                               const int2 *__restrict__ map, int *err,
-                                                              double modfit_bs, double pi, int h1_copies) {
+                                                              const __grid_constant__ Consts c, int h1_copies) {
     const int2 m = map[blockIdx.x];
     const PrepDesc &d = sys[m.x];
-    prep_body<T>(d.geo, d.cols[0], d.cols[1], d.cols[2], d.ld, d.prec, d.dof, d.bins, err, modfit_bs, pi, m.y,
-                   h1_copies);
+    prep_body<T>(d.geo, d.cols[0], d.cols[1], d.cols[2], d.ld, d.prec, d.dof, d.bins, err, c, m.y, h1_copies);
 }
 
 __global__ void nlogn_kernel(double *t, int nmax) {
@@ -596,36 +615,45 @@ size_t prep_smem_bytes(const SysGeom &g) {
     return ((size_t)kWarps * (kModfitBins + m2) + (size_t)c1 * m1) * sizeof(unsigned int);
 }
 
+static Consts prep_consts() {
+    Consts c;
+    c.pi = acos(-1.0);                                                // PARENT.cpp:112
+    c.modfit_bs = (2 * c.pi + 0.000000005) / kModfitBins;  // PARENT.cpp:569
+    c.rm = (float)(1.0 / c.modfit_bs);
+    c.r2pi = (float)(1.0 / (2 * c.pi));
+    c.tp2.hi = (float)(2 * c.pi);
+    c.tp2.lo = (float)(2 * c.pi - (double)c.tp2.hi);
+    return c;
+}
+
 cudaError_t launch_prep(const SysGeom &g, const void *const cols[3], int64_t ld, int double_prec,
                         DofArrays dof, uint8_t *bins, int *err, cudaStream_t st, int g_first, int g_count) {
     if (g_count < 0) g_count = g.D - g_first;
     if (g_first < 0 || g_first + g_count > g.D) return cudaErrorInvalidValue;
     if (g_count == 0) return cudaSuccess;
-    const double pi = acos(-1.0);  // PARENT.cpp:112
-    const double modfit_bs = (2 * pi + 0.000000005) / kModfitBins;  // PARENT.cpp:569
+    const Consts c = prep_consts();
     const size_t smem = prep_smem_bytes(g);
     auto kern = double_prec ? prep_kernel<double> : prep_kernel<float>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int m1 = 0, m2 = 0;
     const int c1 = prep_h1_copies(g, &m1, &m2);
-    kern<<<g_count, kThreads, smem, st>>>(g, cols[0], cols[1], cols[2], ld, double_prec, dof, bins, err, modfit_bs,
-                                          pi, g_first, c1);
+    kern<<<g_count, kThreads, smem, st>>>(g, cols[0], cols[1], cols[2], ld, double_prec, dof, bins, err, c, g_first,
+                                          c1);
     return cudaGetLastError();
 }
 
 cudaError_t launch_prep_batch(const SysGeom &bins_of, const PrepDesc *sys, const int2 *map, int n_cta,
                               int double_prec, int *err, cudaStream_t st) {
     if (n_cta <= 0) return cudaSuccess;
-    const double pi = acos(-1.0);  // PARENT.cpp:112
-    const double modfit_bs = (2 * pi + 0.000000005) / kModfitBins;  // PARENT.cpp:569
+    const Consts c = prep_consts();
     const size_t smem = prep_smem_bytes(bins_of);
     int m1 = 0, m2 = 0;
     const int c1 = prep_h1_copies(bins_of, &m1, &m2);
     auto kern = double_prec ? prep_batch_kernel<double> : prep_batch_kernel<float>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<n_cta, kThreads, smem, st>>>(sys, map, err, modfit_bs, pi, c1);
+    kern<<<n_cta, kThreads, smem, st>>>(sys, map, err, c, c1);
     return cudaGetLastError();
 }
 
