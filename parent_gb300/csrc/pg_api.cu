@@ -1174,11 +1174,16 @@ PG_API int pg_entropy(pg_ctx *ctx, const pg_bat_view *traj, const int bins[6], i
             if (rch) return rch;
         }
     } else {
-        const size_t sb = pairs_onehot_scratch_bytes(g);
+        bool bits = onehot_bits({g});
+        if (bits && ctx->scratch.ensure(pairs_onehot_scratch_bytes(g, true)) != cudaSuccess) {
+            cudaGetLastError();  // no memory for the masks: the FP8 kernel needs none
+            bits = false;
+        }
+        const size_t sb = pairs_onehot_scratch_bytes(g, bits);
         CK(ctx->scratch.ensure(sb));
         int nl = 0;
         CK(launch_pairs_onehot(g, (const uint8_t *)ctx->bins.p, dof, (const double *)ctx->nlogn.p, po,
-                               (int *)ctx->errw.p, st, ctx->scratch.p, sb, &nl));
+                               (int *)ctx->errw.p, st, ctx->scratch.p, sb, bits, &nl));
         ctx->launches += nl;
     }
     ctx->last_form = chosen;
@@ -1862,7 +1867,12 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
         tiles.insert(tiles.end(), t.begin(), t.end());
         tsys.insert(tsys.end(), t.size(), s);
     }
-    if (onehot) CK(ctx->ohbatch.ensure(pairs_onehot_batch_bytes(gs)));
+    bool obits = onehot && onehot_bits(gs);
+    if (obits && ctx->ohbatch.ensure(pairs_onehot_batch_bytes(gs, true)) != cudaSuccess) {
+        cudaGetLastError();  // no memory for the masks: the FP8 kernel needs none
+        obits = false;
+    }
+    if (onehot) CK(ctx->ohbatch.ensure(pairs_onehot_batch_bytes(gs, obits)));
     // preprocessing of all systems in one launch per input precision: CTA
     // k handles DOF map[k].y of system map[k].x
     std::vector<PrepDesc> pd((size_t)n_sys);
@@ -1915,6 +1925,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
     key.push_back(sys[0].g.codes);
     key.push_back(sys[0].g.ilv);
     key.push_back(onehot ? (int64_t)(uintptr_t)ctx->ohbatch.p : -1);
+    key.push_back(obits);
     key.push_back(srt ? (int64_t)(uintptr_t)ctx->sscr.p : -1);
     key.push_back(tree);
     key.push_back(joint);
@@ -1957,7 +1968,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
                 dp[s] = sd[s].dof;
                 op[s] = sd[s].out;
             }
-            CK(prepare_pairs_onehot_batch(gs, bp, dp, op, ctx->ohbatch.p, ctx->ohbatch.n, st));
+            CK(prepare_pairs_onehot_batch(gs, bp, dp, op, ctx->ohbatch.p, ctx->ohbatch.n, obits, st));
             ctx->launches += n_sys;  // one n ln n table per system
         }
     }
@@ -2004,7 +2015,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
         }
         int oh_launches = 0, tree_launches = 0;
         if (e == cudaSuccess && onehot)
-            e = launch_pairs_onehot_batch(gs, ctx->ohbatch.p, (int *)ctx->errw.p, st, &oh_launches);
+            e = launch_pairs_onehot_batch(gs, ctx->ohbatch.p, obits, (int *)ctx->errw.p, st, &oh_launches);
         else if (e == cudaSuccess && srt) {
             SortedArgs a{};
             a.many = (const SortedSys *)(meta + mo_so);
@@ -2049,7 +2060,7 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
     }
     CK(cudaGraphLaunch(ctx->graph, st));
     // preps, pair kernel (+ the one-hot finalize), MIST
-    ctx->launches += ctx->graph_tree_launches + (pmap[0].empty() ? 0 : 1) + (pmap[1].empty() ? 0 : 1) + (onehot ? 3 : (srt ? 5 : 2));
+    ctx->launches += ctx->graph_tree_launches + (pmap[0].empty() ? 0 : 1) + (pmap[1].empty() ? 0 : 1) + (onehot ? (obits ? 4 : 3) : (srt ? 5 : 2));
     CK(cudaEventRecord(ctx->ev[2], st));
     int rc = check_err_words(ctx);
     float ms[2];

@@ -4,13 +4,13 @@
 // Both forms walk a tile list with a fixed amount of work per tile and frame:
 //   - the histogram kernels are persistent (one CTA per SM strides over the
 //     tiles), so a launch takes ceil(tiles / grid) tile times;
-//   - the one-hot kernel runs one CTA pair per 256 x 512 block of C, two
-//     SMs each, so a launch takes ceil(tiles / (SMs / 2)) tile times.
+//   - the one-hot kernels run one CTA pair per 256 x 448 (FP8: 256 x 512) block
+//     of C, two SMs each, so a launch takes ceil(tiles / (SMs / 2)) tile times.
 // A tile time is t0 + t1 * F (t0: per-tile set-up and epilogue; t1: the frame
 // loop). The tile counts come from the geometry (D and the bin counts: the
-// one-hot form has one tile per 256 x 512 block of the (DOF, bin) space, so
+// one-hot form has one tile per block of the (DOF, bin) space, so
 // its tile count grows as B^2), the constants from two probe launches per
-// kernel (F = 4,096 and 32,768 frames, random bins, at least one full wave of
+// kernel (F = 4,096 and 16,384 or 32,768 frames, random bins, at least one full wave of
 // tiles), measured once per process, device and kernel variant. The form with
 // the smaller predicted time is picked; when probing is not possible the
 // measured crossover (one-hot up to 15 bins, from 4,096 frames) decides.
@@ -50,7 +50,8 @@ struct TileCost {
     bool ok = false;
 };
 
-// key: (device, kernel variant: 0 one-hot, 1 + layout, bmax)
+// key: (device, kernel variant, bmax)
+constexpr int kOnehotBits = -1, kOnehot = 0, kHist = 1;  // kHist + layout
 std::mutex g_mu;
 std::map<std::tuple<int, int, int>, TileCost> g_costs;
 
@@ -141,13 +142,14 @@ cudaError_t time_launch(Probe &p, int variant, cudaStream_t st, double *sec, dou
     std::vector<PairTile> tl;
     void *dtiles = nullptr;
     int T = 0, fc = 0, nst = 0;
-    if (variant == 0) {
-        const size_t sb = pairs_onehot_scratch_bytes(g);
+    const bool bits = variant == kOnehotBits;
+    if (variant <= kOnehot) {
+        const size_t sb = pairs_onehot_scratch_bytes(g, bits);
         if ((e = p.alloc(&p.scratch, sb))) return e;
         p.scratch_bytes = sb;
-        *waves = ceil((double)pairs_onehot_tiles(g) / std::max(1, sms / 2));
+        *waves = ceil((double)pairs_onehot_tiles(g, bits) / std::max(1, sms / 2));
     } else {
-        if (variant - 1 == 0) {
+        if (variant - kHist == HIST16) {
             if (!pairs_hist_config(bmax_of(g), &T, &fc, &nst)) return cudaErrorInvalidValue;
             tl = build_tiles(g.D, T);
         } else {
@@ -165,14 +167,14 @@ cudaError_t time_launch(Probe &p, int variant, cudaStream_t st, double *sec, dou
     const double fix = nlogn_fix_scale(g.F);
     OnehotRun run;
     *setup = 0.0;
-    if (variant == 0) {
+    if (variant <= kOnehot) {
         const auto t0 = std::chrono::steady_clock::now();
-        if ((e = onehot_setup(g, p.bins, p.dof, p.out, st, p.scratch, p.scratch_bytes, &run))) return e;
+        if ((e = onehot_setup(g, p.bins, p.dof, p.out, st, p.scratch, p.scratch_bytes, bits, &run))) return e;
         *setup = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     }
     auto launch = [&]() -> cudaError_t {
-        if (variant == 0) return onehot_run(run, p.err, st);
-        if (variant - 1 == 0)
+        if (variant <= kOnehot) return onehot_run(run, p.err, st);
+        if (variant - kHist == HIST16)
             return launch_pairs_hist(g, p.bins, p.dof, p.nfix, fix, (const PairTile *)dtiles, (int64_t)tl.size(), T,
                                      p.out, p.err, st);
         return launch_pairs_hist32(g, p.bins, p.dof, p.nfix, fix, (const PairTile *)dtiles, (int64_t)tl.size(),
@@ -202,10 +204,11 @@ TileCost calibrate(const SysGeom &like, int variant) {
     TileCost c;
     const int sms = sm_count_now();
     int D;
-    if (variant == 0) {
-        // at least one full wave of CTA pairs: R = D B rows, tiles ~ R^2 / (2 256 512)
+    if (variant <= kOnehot) {
+        // more than two waves of CTA pairs (what a call costs once counts little):
+        // R = D B rows, tiles ~ R^2 / (2 256 512)
         const int B = bmax_of(like);
-        const double R = sqrt(2.0 * 256.0 * 512.0 * (sms / 2) * 1.2);
+        const double R = sqrt(2.0 * 256.0 * 512.0 * (sms / 2) * 2.4);
         D = std::max(96, (int)ceil(R / B));
     } else {
         D = 3 * 60;  // 180 DOFs: ~2 waves of 32-slot tiles, ~7 of 16-slot tiles on 152 SMs
@@ -216,7 +219,7 @@ TileCost calibrate(const SysGeom &like, int variant) {
         cudaGetLastError();
         return c;
     }
-    const int Fs[2] = {4096, 32768};
+    const int Fs[2] = {4096, variant <= kOnehot ? 16384 : 32768};
     double t[2] = {0, 0}, setup = 0.0;
     bool ok = true;
     for (int k = 0; k < 2 && ok; k++) {
@@ -243,7 +246,7 @@ TileCost cost_of(const SysGeom &g, int variant) {
     cudaGetDevice(&dev);
     // the one-hot tile costs the same at any bin count; histogram tiles
     // depend on the layout and the bin count
-    const auto key = std::make_tuple(dev, variant, variant == 0 ? 0 : bmax_of(g));
+    const auto key = std::make_tuple(dev, variant, variant <= kOnehot ? 0 : bmax_of(g));
     {
         std::lock_guard<std::mutex> lock(g_mu);
         auto it = g_costs.find(key);
@@ -364,15 +367,16 @@ double predict_pair_seconds(const SysGeom &g, int form) {
     if (form == PG_FORM_ONEHOT) {
         if (!pairs_onehot_supported(g)) return -1.0;
         const SysGeom h = as_onehot(g);
-        const TileCost c = cost_of(h, 0);
+        const bool bits = onehot_bits({g});
+        const TileCost c = cost_of(h, bits ? kOnehotBits : kOnehot);
         if (!c.ok) return -1.0;
-        const double waves = ceil((double)pairs_onehot_tiles(h) / std::max(1, sms / 2));
+        const double waves = ceil((double)pairs_onehot_tiles(h, bits) / std::max(1, sms / 2));
         return c.call + waves * (c.t0 + c.t1 * g.F);
     }
     if (sorted_layout({g})) return sum_sorted({g}, sorted_joint({g}));
     const int layout = hist_layout(g);
     const SysGeom h = as_hist(g, layout);
-    const TileCost c = cost_of(h, 1 + (layout == HIST16 ? 0 : layout));
+    const TileCost c = cost_of(h, kHist + layout);
     if (!c.ok) return -1.0;
     int64_t tiles;
     if (layout == HIST16) {
@@ -413,11 +417,11 @@ int autotune_batch_form(const std::vector<SysGeom> &gs) {
             if (!fallback_onehot(g)) return PG_FORM_HIST;
         return PG_FORM_ONEHOT;
     }
-    const bool sorted = sorted_layout(gs), joint = sorted && sorted_joint(gs);
+    const bool bits = onehot_bits(gs), sorted = sorted_layout(gs), joint = sorted && sorted_joint(gs);
     for (const SysGeom &g : gs) {
         const int layout = hist_layout(g);
-        const TileCost ch = sorted ? TileCost{} : cost_of(as_hist(g, layout), 1 + (layout == HIST16 ? 0 : layout));
-        const TileCost co = cost_of(as_onehot(g), 0);
+        const TileCost ch = sorted ? TileCost{} : cost_of(as_hist(g, layout), kHist + layout);
+        const TileCost co = cost_of(as_onehot(g), bits ? kOnehotBits : kOnehot);
         if ((!sorted && !ch.ok) || !co.ok) {
             for (const SysGeom &x : gs)
                 if (!fallback_onehot(x)) return PG_FORM_HIST;
@@ -434,7 +438,7 @@ int autotune_batch_form(const std::vector<SysGeom> &gs) {
         // one launch for the whole batch (its set-up runs once, outside the
         // replayed graph)
         th += sorted ? sorted_seconds(g, joint) : (double)tiles * (ch.t0 + ch.t1 * g.F) / sms;
-        to += (double)pairs_onehot_tiles(as_onehot(g)) * (co.t0 + co.t1 * g.F) / std::max(1, sms / 2);
+        to += (double)pairs_onehot_tiles(as_onehot(g), bits) * (co.t0 + co.t1 * g.F) / std::max(1, sms / 2);
     }
     return to < th ? PG_FORM_ONEHOT : PG_FORM_HIST;
 }

@@ -354,8 +354,11 @@ cudaError_t launch_mie_compact(const MieArgs &a, cudaStream_t st);   // slots ->
 // tcgen05 one-hot pair kernel (same outputs as the histogram kernel).
 cudaError_t launch_pairs_onehot(const SysGeom &g, const uint8_t *bins, const DofArrays &dof,
                                 const double *nlogn, PairOut out, int *err, cudaStream_t st,
-                                void *scratch, size_t scratch_bytes, int *launches);
-size_t pairs_onehot_scratch_bytes(const SysGeom &g);
+                                void *scratch, size_t scratch_bytes, bool bits, int *launches);
+// bits: the kernel that reads one-bit masks, where onehot_bits allows it for
+// all systems of a launch (its scratch holds the masks).
+bool onehot_bits(const std::vector<SysGeom> &gs);
+size_t pairs_onehot_scratch_bytes(const SysGeom &g, bool bits);
 bool pairs_onehot_supported(const SysGeom &g);
 // launch_pairs_onehot in two parts: the set-up (synchronous uploads, the
 // n ln n table) and the run (accumulators zeroed, pair kernel, finalize),
@@ -364,12 +367,12 @@ struct OnehotRun {
     void *scratch = nullptr;
     size_t off_sys = 0, off_fin = 0, off_tiles = 0, off_snl = 0, acc_bytes = 0;
     int64_t n_tiles = 0;
-    bool pair = true;
+    int kind = 0;
     bool low = false;  // every 2D bin count at most 64
-    int D = 0;
+    int D = 0, F = 0;
 };
 cudaError_t onehot_setup(const SysGeom &g, const uint8_t *bins, const DofArrays &dof, PairOut out, cudaStream_t st,
-                         void *scratch, size_t scratch_bytes, OnehotRun *run);
+                         void *scratch, size_t scratch_bytes, bool bits, OnehotRun *run);
 cudaError_t onehot_run(const OnehotRun &run, int *err, cudaStream_t st);
 // Many systems in one one-hot launch (each tile names its system; tiles of
 // the longest trajectories first): workspace size, tile count, the set-up
@@ -377,12 +380,11 @@ cudaError_t onehot_run(const OnehotRun &run, int *err, cudaStream_t st);
 // (synchronous, outside any graph capture), and the launch itself (zeroes
 // the accumulators, pair kernel, one finalize launch over all systems;
 // capturable).
-size_t pairs_onehot_batch_bytes(const std::vector<SysGeom> &gs);
-int64_t pairs_onehot_batch_tiles(const std::vector<SysGeom> &gs);
+size_t pairs_onehot_batch_bytes(const std::vector<SysGeom> &gs, bool bits);
 cudaError_t prepare_pairs_onehot_batch(const std::vector<SysGeom> &gs, const std::vector<const uint8_t *> &bins,
                                        const std::vector<DofArrays> &dofs, const std::vector<PairOut> &outs,
-                                       void *ws, size_t ws_bytes, cudaStream_t st);
-cudaError_t launch_pairs_onehot_batch(const std::vector<SysGeom> &gs, void *ws, int *err, cudaStream_t st,
+                                       void *ws, size_t ws_bytes, bool bits, cudaStream_t st);
+cudaError_t launch_pairs_onehot_batch(const std::vector<SysGeom> &gs, void *ws, bool bits, int *err, cudaStream_t st,
                                       int *launches);
 
 // One system of a MIST launch. scratch: mist_tree_bytes(D) for the tree
@@ -411,9 +413,8 @@ cudaError_t launch_mi_from_par(int n_dih, const double *par, ParLayout L, double
                                cudaStream_t st);
 
 std::vector<PairTile> build_tiles32(int D);
-// tile count of the one-hot form for a geometry (CTA-pair tiles unless
-// PG_ONEHOT_PAIR=0)
-int64_t pairs_onehot_tiles(const SysGeom &g);
+// tile count of the one-hot form for a geometry
+int64_t pairs_onehot_tiles(const SysGeom &g, bool bits);
 
 // Histogram layouts: the 16-slot kernel (two lanes per pair), the 32-slot
 // kernel fed by a TMA ring, and the streamed 32-slot kernel (rows loaded

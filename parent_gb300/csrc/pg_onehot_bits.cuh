@@ -1,0 +1,401 @@
+// One-hot pair kernel on packed FP4 operands, built from one-bit masks. A part
+// of pg_pairs_onehot.cu (its helpers, OhSys, TcTile), inside its namespace.
+//
+// onehot_bits_kernel writes X itself, one bit an entry: per 256-frame K-block
+// and row of C eight words. The pair kernel's builders only spread bits over
+// nibbles. A word m of 32 frames gives four operand words, one per bit of a
+// nibble; an E2M1 nibble is 0.5, 1 or 2 by its one set bit among the lower
+// three, so of most bits the mask alone is the operand, and what A holds as
+// 0.5, 1, 2, 2 the same frames of B hold as 2, 1, 0.5, 0.5: every product is 1
+// and the FP32 accumulators hold counts. All scale factors are 1 (0x7f), so
+// which word of tensor memory scales which block does not matter.
+//
+// What bounds it: the tensor pipe, at twice the FP8 rate, and next to it shared
+// memory: a K-block of 256 frames takes 896 cycles of MMAs (128 x 448 x 256 a
+// CTA), 480 of their operand reads and 352 of the builders' stores, and 280 of
+// ALU work (five to seven operations per 32 frames and row; bytes compared
+// with a bin take 24). Measured 0.51 us (1,000 cycles) a K-block, and 11 us a
+// tile around them. 2,994 DOFs x 100k frames x 10 bins: 36.2 -> 11.8 ms. What
+// the FP8 kernel and first versions of this one lost:
+//   - one warp relaying every stage to the first CTA, at 1,500 cycles each: a
+//     relay warp per stage (0.73 -> 0.64 us a K-block);
+//   - the issuer's lane waiting for its warp and making descriptors per MMA: one
+//     lane, unrolled over the stages (0.64 -> 0.54);
+//   - masks read as two 16-byte halves: 32-byte loads (0.54 -> 0.51); without
+//     any load 0.46, the tensor pipe's own time;
+//   - counts looked up in global memory and summed by shared atomics: a copy of
+//     the table and partial sums in shared memory (40 -> 19 us a tile).
+// Five stages, two builder groups in turn and 128-byte swizzled operands were
+// within 2 %.
+// Tile 256 x 448: the scale factors take 64 of the 512 columns of tensor
+// memory. Four stages of 44 KB; a thread owns one operand row and has its masks
+// of three K-blocks in flight.
+
+constexpr int kBitN = 448, kBitNH = 224;           // tile columns, N of one MMA
+constexpr int kBitKB = 256;                        // frames per K-block (128 bytes a row)
+constexpr int kBitBRows = kBitN / 2;               // B rows built by a CTA
+constexpr int kBitBuilders = (kM + kBitBRows) / 32;  // warps, one row a thread
+constexpr int kBitIssuer = kBitBuilders;           // the warp that issues the MMAs
+constexpr int kBitStages = 4;
+constexpr int kBitThreads = (kBitIssuer + 1 + kBitStages + 3) / 4 * 128;  // and a relay warp per stage
+constexpr int kBitStageBytes = (kM + kBitBRows) * 128;
+constexpr int kBitScaleCol = kBitN;                // tensor memory columns of the scale factors
+constexpr int kBitMaxFrames = 1 << 22;             // of a launch: accumulators far inside FP32's 2^24
+constexpr int kBitOffBar = kBitStages * kBitStageBytes;  // full[kBitStages] | empty[kBitStages]
+constexpr int kBitOffTmem = kBitOffBar + 2 * kBitStages * 8;
+constexpr int kBitSmem = kBitOffTmem + 16;
+// epilogue: the columns in kBitParts parts, partial sums [part][slot][row] and
+// the first entries of the n ln n table in the stages, a slot per DOF of the
+// part's columns (2D bins >= 8)
+constexpr int kBitParts = kBitThreads / 128, kBitChunks = kBitN / 16;
+constexpr int kBitSlots = ((kBitChunks + kBitParts - 1) / kBitParts * 16 - 1) / 8 + 2;
+static_assert((kM + kBitBRows) % 32 == 0 && kBitNH / 2 % 8 == 0 && kBitSmem <= 227 * 1024, "");
+constexpr int kBitLd = kM + 1, kBitLdOcc = kM + 4;  // slot strides, in values and bytes: odd in banks
+constexpr int kBitTable = (kBitOffBar - kBitParts * kBitSlots * (kBitLd * 8 + kBitLdOcc)) / 8 / 128 * 128;  // n ln n
+static_assert(kBitTable >= 8192, "");
+
+// D = F32, A = B = E2M1 (1), UE8M0 scale factors (bit 23), both K-major, K = 64
+constexpr uint32_t kIdescBits = (1u << 7) | (1u << 10) | ((uint32_t)(kBitNH >> 3) << 17) | (1u << 23) |
+                                ((uint32_t)((2 * kM) >> 4) << 24);
+
+__device__ __forceinline__ void mma_f4_pair(uint32_t tmem, uint64_t adesc, uint64_t bdesc, uint32_t acc,
+                                            uint32_t scales) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], p;\n\t}" ::"r"(
+            tmem),
+        "l"(adesc), "l"(bdesc), "r"(kIdescBits), "r"(acc), "r"(scales), "r"(scales + 32)
+        : "memory");
+}
+
+// first row of DOF d in C
+__device__ __forceinline__ int bits_first_row(const OhSys &sy, int d) {
+    const int nba = sy.nb + sy.na;
+    return min(d, sy.nb) * sy.b2[TB] + max(0, min(d, nba) - sy.nb) * sy.b2[TA] + max(0, d - nba) * sy.b2[TD];
+}
+
+// The masks of DOF blockIdx.y of system blockIdx.z, 32 frames a thread: the
+// bins' bit planes (frame 4 i + k of the 32 is bit 8 k + i), the eight
+// combinations of the lowest three, each with the higher planes'. Bounded by
+// what it reads and writes: 1 + B / 8 bytes a value.
+__global__ void __launch_bounds__(256) onehot_bits_kernel(const OhSys *__restrict__ systems) {
+    const OhSys &sy = systems[blockIdx.z];
+    const int d = blockIdx.y, t = blockIdx.x * 256 + threadIdx.x;
+    if (d >= sy.D || t >= (sy.F + kBitKB - 1) / kBitKB * 8) return;
+    const int B = sy.b2[dof_type(d, sy.nb, sy.na)], row = bits_first_row(sy, d);
+    const uint4 *p = (const uint4 *)(sy.bins + (int64_t)d * sy.ldb + (int64_t)t * 32);
+    const uint4 u = __ldg(p), v = __ldg(p + 1);
+    const uint32_t w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+    const int np = 32 - __clz(B - 1);
+    uint32_t pl[7];
+#pragma unroll
+    for (int q = 0; q < 7; q++) {
+        pl[q] = 0u;
+        if (q < np) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) pl[q] |= (i >= q ? w[i] << (i - q) : w[i] >> (q - i)) & (0x01010101u << i);
+        }
+    }
+    uint32_t vm = 0xffffffffu;
+    const int left = sy.F - t * 32;
+    if (left < 32) {  // frames past F are no data
+        vm = 0u;
+        for (int f = 0; f < left; f++) vm |= 1u << (8 * (f & 3) + (f >> 2));
+    }
+    uint32_t low[8];
+#pragma unroll
+    for (int l = 0; l < 8; l++) low[l] = (l & 1 ? pl[0] : ~pl[0]) & (l & 2 ? pl[1] : ~pl[1]) & (l & 4 ? pl[2] : ~pl[2]);
+    uint32_t *out = sy.bits + ((int64_t)(t >> 3) * sy.R + row) * 8 + (t & 7);
+    for (int h = 0; 8 * h < B; h++) {
+        uint32_t hm = vm;
+#pragma unroll
+        for (int q = 3; q < 7; q++)
+            if (q < np) hm &= (h >> (q - 3)) & 1 ? pl[q] : ~pl[q];
+#pragma unroll
+        for (int l = 0; l < 8; l++)
+            if (8 * h + l < B) out[(8 * h + l) * 8] = low[l] & hm;
+    }
+}
+
+// A CTA pair (cluster of 2) computes the 256 x 448 tile (mt, nt) of C: CTA
+// `rank` owns rows 256 mt + 128 rank .. +127 and, of each 224-column MMA, B
+// columns 112 rank .. +111. Roles, barriers and the epilogue as in
+// onehot_kernel: builder warps arrive on their CTA's "full" barrier, the last
+// warp of rank 1 relays to rank 0, whose last warp issues the stage's eight
+// MMAs and commits them to "empty" in both CTAs. Every wait is bounded.
+__global__ void __launch_bounds__(kBitThreads, 1)
+onehot_bits_pairs_kernel(const OhSys *__restrict__ systems, const TcTile *__restrict__ tiles, int *err) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    uint64_t *full = (uint64_t *)(smem + kBitOffBar), *empty = full + kBitStages;
+    uint32_t *tmem_slot = (uint32_t *)(smem + kBitOffTmem);
+    __shared__ __align__(16) int s_cdof[kBitN];  // DOF of each column of the tile (-1 past R)
+    __shared__ int s_mma_issued;
+    __shared__ volatile int s_abort;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t rank = cluster_rank();
+    const TcTile tile = tiles[blockIdx.x >> 1];
+    const OhSys &sy = systems[tile.sys];
+    const uint32_t *__restrict__ rowinfo = sy.rowinfo;
+    const int R = sy.R, nkb = (sy.F + kBitKB - 1) / kBitKB;
+    const int r0 = tile.mt * 2 * kM + (int)rank * kM, c0 = tile.nt * kBitN;
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    for (int c = tid; c < kBitN; c += kBitThreads) s_cdof[c] = c0 + c < R ? (int)(rowinfo[c0 + c] >> 8) : -1;
+    if (tid == 0) {
+        for (int k = 0; k < kBitStages; k++) {
+            mbar_init(smem_u32(&full[k]), rank == 0 ? kBitBuilders + 1 : kBitBuilders);
+            mbar_init(smem_u32(&empty[k]), 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_abort = 0;
+        s_mma_issued = 0;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+    if (warp < 4) {  // a warp writes its quarter of the lanes
+        for (int c = kBitScaleCol; c < 512; c += 8)
+            asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(
+                             tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c),
+                         "r"(0x7f7f7f7fu)
+                         : "memory");
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    cluster_sync_all();  // scale factors and barriers of both CTAs before the first MMA or remote arrival
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+    if (warp == kBitIssuer) {
+        if (rank == 0) {
+            // --------------------------------------------------- MMA issuer
+            if (lane == 0) {
+                const uint64_t ad = smem_desc(smem_u32(smem), 128, 1024), bd = smem_desc(smem_u32(smem) + kAStage, 128, 1024);
+                int done = 0;
+                bool go = true;
+                for (int k0 = 0; k0 < nkb && go; k0 += kBitStages) {
+                    const uint32_t parity = (uint32_t)((k0 / kBitStages) & 1);
+                    if (s_abort) break;
+#pragma unroll
+                    for (int s = 0; s < kBitStages; s++) {
+                        if (k0 + s >= nkb) break;
+                        if (!mbar_wait_cluster_bounded(smem_u32(&full[s]), parity)) {
+                            s_abort = 1;
+                            go = false;
+                            break;
+                        }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                        for (int kk = 0; kk < 4; kk++) {
+#pragma unroll
+                            for (int h = 0; h < 2; h++)  // 16-byte units of the descriptors' addresses
+                                mma_f4_pair(tmem + h * kBitNH, ad + (s * kBitStageBytes + kk * 256) / 16,
+                                            bd + (s * kBitStageBytes + h * (kBitNH / 2) * 128 + kk * 256) / 16,
+                                            (k0 | s | kk) != 0, tmem + kBitScaleCol);
+                        }
+                        mma_commit_pair(smem_u32(&empty[s]));
+                        done++;
+                    }
+                }
+                s_mma_issued = done;
+            }
+            __syncwarp();
+        }
+    } else if (warp > kBitIssuer) {
+        if (rank == 1) {
+            // ------------------------------------------ rank 1: stage relay
+            const int s = warp - kBitIssuer - 1;
+            const uint32_t full_c0 = map_to_rank(smem_u32(&full[0]), 0u) + (uint32_t)s * 8u;
+            for (int kb = s; kb < nkb && s < kBitStages; kb += kBitStages) {
+                int ok = 1;
+                if (lane == 0) ok = mbar_wait_bounded(smem_u32(&full[s]), (uint32_t)((kb / kBitStages) & 1)) ? 1 : 0;
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (!ok || s_abort) {
+                    if (lane == 0) s_abort = 1;
+                    break;
+                }
+                if (lane == 0) mbar_arrive_cluster(full_c0);
+                __syncwarp();
+            }
+        }
+    } else {
+        // ----------------------------------------------------------- builders
+        const bool isA = tid < kM;  // the same for a warp
+        const int i = isA ? tid : tid - kM, h = i / (kBitNH / 2);
+        const int row = isA ? r0 + i : c0 + h * kBitNH + (int)rank * (kBitNH / 2) + i % (kBitNH / 2);
+        // 8 rows x 16 bytes are contiguous (a core matrix), 8 of them a group of 8 rows
+        unsigned char *dst = smem + (isA ? 0 : kAStage) + (i >> 3) * 1024 + (i & 7) * 16;
+        const uint4 *src = (const uint4 *)(sy.bits + (int64_t)row * 8);
+        const int64_t step = (int64_t)R * 2;  // a K-block of masks, in uint4
+        const bool live = row < R;
+        // the masks of the next three K-blocks in flight; the loop is unrolled
+        // over the stages so that no load is waited for early
+        uint4 buf[kBitStages][2];
+        auto load = [&](int kb, uint4 *v) {
+            v[0] = v[1] = make_uint4(0u, 0u, 0u, 0u);
+            if (live && kb < nkb) {
+                asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                             : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w), "=r"(v[1].x), "=r"(v[1].y),
+                               "=r"(v[1].z), "=r"(v[1].w)
+                             : "l"(src + kb * step));
+            }
+        };
+#pragma unroll
+        for (int u = 0; u < kBitStages - 1; u++) load(u, buf[u]);
+        bool go = true;
+        for (int k0 = 0; k0 < nkb && go; k0 += kBitStages) {
+            const uint32_t parity = (uint32_t)((k0 / kBitStages - 1) & 1);
+            if (s_abort) break;
+#pragma unroll
+            for (int s = 0; s < kBitStages; s++) {
+                if (k0 + s >= nkb) break;
+                load(k0 + s + kBitStages - 1, buf[(s + kBitStages - 1) % kBitStages]);
+                if (k0 > 0 && !mbar_wait_bounded(smem_u32(&empty[s]), parity)) {
+                    s_abort = 1;
+                    go = false;
+                    break;
+                }
+                const uint32_t m[8] = {buf[s][0].x, buf[s][0].y, buf[s][0].z, buf[s][0].w,
+                                       buf[s][1].x, buf[s][1].y, buf[s][1].z, buf[s][1].w};
+                unsigned char *st = dst + s * kBitStageBytes;
+                if (isA) {
+#pragma unroll
+                    for (int c = 0; c < 8; c++)
+                        *(uint4 *)(st + c * 128) = make_uint4(m[c] & 0x11111111u, m[c] & 0x22222222u,
+                                                              m[c] & 0x44444444u, m[c] >> 1 & 0x44444444u);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 8; c++)
+                        *(uint4 *)(st + c * 128) = make_uint4(m[c] << 2 & 0x44444444u, m[c] & 0x22222222u,
+                                                              m[c] >> 2 & 0x11111111u, m[c] >> 3 & 0x11111111u);
+                }
+                // generic writes of the stage before the tensor core reads it
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&full[s]));
+            }
+        }
+    }
+    __syncthreads();
+
+    bool aborted = s_abort != 0;
+    if (!aborted && nkb > 0) {  // the commit of the final block covers every earlier MMA
+        const int last = nkb - 1;
+        if (!mbar_wait_bounded(smem_u32(&empty[last % kBitStages]), (uint32_t)((last / kBitStages) & 1))) s_abort = 1;
+        aborted = __syncthreads_or(s_abort != 0);
+    }
+    if (aborted) {
+        // record it, let issued MMAs finish (bounded), free the tensor memory
+        if (tid == 0) {
+            atomicAdd(&err[ERR_TIMEOUT], 1);
+            const int nm = s_mma_issued;
+            for (int k = nm > kBitStages ? nm - kBitStages : 0; k < nm; k++)
+                (void)mbar_wait_bounded(smem_u32(&empty[k % kBitStages]), (uint32_t)((k / kBitStages) & 1));
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        cluster_sync_all();  // neither CTA leaves while the pair's MMAs may read its stages
+        if (warp == 0)
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+        return;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+    // ---- epilogue: warp w reads lanes 32 (w % 4).. and a part of the columns.
+    // A thread sums its row per column DOF into the part's slots; then one
+    // thread per (row DOF, slot) adds up the DOF's rows. 57,344 counts a CTA, each
+    // a read of the n ln n table, a cycle per line that a warp touches in global
+    // memory: the entries that fit beside the sums (all but the largest counts to
+    // some 100,000 frames) are copied in first. Rows and columns past R have no
+    // bits, so no count, and entry 0 is 0.
+    unsigned long long *ps_snl = (unsigned long long *)smem;  // every MMA has read the stages
+    long long *s_tab = (long long *)(ps_snl + kBitParts * kBitSlots * kBitLd);
+    unsigned char *ps_occ = (unsigned char *)(s_tab + kBitTable);
+    const int row = 32 * (warp & 3) + lane, grow = r0 + row;
+    const int rend = min(R - r0, kM);
+    const int rdof = (int)(rowinfo[min(grow, R - 1)] >> 8);
+    const int part = warp >> 2, ch0 = kBitChunks * part / kBitParts, ch1 = kBitChunks * (part + 1) / kBitParts;
+    const int64_t *__restrict__ nlogn_fix = sy.nfix;
+    const uint32_t ntab = (uint32_t)min(sy.F + 1, kBitTable);
+    for (uint32_t k = tid; k < ntab; k += kBitThreads) s_tab[k] = __ldg(nlogn_fix + k);
+    __syncthreads();
+    int cur = s_cdof[ch0 * 16], slot = part * kBitSlots;
+    // whether some pair of the part is no pair g1 < g2
+    const bool mixed = cur <= (int)(rowinfo[max(0, min(r0 + kM, R) - 1)] >> 8);
+    unsigned long long snl = 0ull;
+    unsigned int occ = 0u;
+    for (int ch = ch0; ch < ch1; ch++) {
+        uint32_t v[16];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+            : "r"(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(ch * 16)));
+        int cdof[16];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int4 c = *(const int4 *)(s_cdof + ch * 16 + 4 * q);
+            cdof[4 * q] = c.x;
+            cdof[4 * q + 1] = c.y;
+            cdof[4 * q + 2] = c.z;
+            cdof[4 * q + 3] = c.w;
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (mixed) {
+#pragma unroll
+            for (int q = 0; q < 16; q++)
+                if (cdof[q] <= rdof) v[q] = 0u;
+        }
+        unsigned long long t[16];
+#pragma unroll
+        for (int q = 0; q < 16; q++) {  // the counts are below 2^23: their bits, after 2^23 is added
+            v[q] = __float_as_uint(__uint_as_float(v[q]) + 8388608.0f) & 0x7fffffu;
+            t[q] = (unsigned long long)(v[q] < ntab ? s_tab[v[q]] : __ldg(nlogn_fix + v[q]));
+        }
+#pragma unroll
+        for (int q = 0; q < 16; q++) {
+            if (cdof[q] != cur) {  // the same for every row
+                ps_snl[slot * kBitLd + row] = snl;
+                ps_occ[slot * kBitLdOcc + row] = (unsigned char)occ;
+                slot++;
+                cur = cdof[q];
+                snl = 0ull;
+                occ = 0u;
+            }
+            snl += t[q];
+            occ += v[q] != 0u;
+        }
+    }
+    ps_snl[slot * kBitLd + row] = snl;
+    ps_occ[slot * kBitLdOcc + row] = (unsigned char)occ;
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    cluster_sync_all();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    // tile partials -> per-pair accumulators (integer adds: order-independent)
+    if (rend <= 0) return;
+    const int rdof0 = (int)(rowinfo[r0] >> 8), nr = (int)(rowinfo[r0 + rend - 1] >> 8) - rdof0 + 1;
+    for (int e = tid; e < nr * kBitParts * kBitSlots; e += kBitThreads) {
+        const int g1 = rdof0 + e / (kBitParts * kBitSlots), sl = e % (kBitParts * kBitSlots), p = sl / kBitSlots;
+        const int cf = s_cdof[kBitChunks * p / kBitParts * 16], cl = s_cdof[kBitChunks * (p + 1) / kBitParts * 16 - 1];
+        const int g2 = cf + sl % kBitSlots;
+        // the part's last DOF, or the system's where the part passes the last row of C
+        if (cf < 0 || g2 > (cl < 0 ? sy.D - 1 : cl) || g2 <= g1) continue;
+        const int s0 = max(0, bits_first_row(sy, g1) - r0), s1 = min(rend, bits_first_row(sy, g1 + 1) - r0);
+        unsigned long long sum = 0ull;
+        unsigned int o = 0u;
+        for (int r = s0; r < s1; r++) {
+            sum += ps_snl[sl * kBitLd + r];
+            o += ps_occ[sl * kBitLdOcc + r];
+        }
+        if (!o) continue;
+        atomicAdd(&sy.acc_snl[(int64_t)g1 * sy.D + g2], sum);
+        atomicAdd(&sy.acc_occ[(int64_t)g1 * sy.D + g2], o);
+    }
+}

@@ -29,6 +29,7 @@
 // pair's accumulators. Integer atomics keep the result independent of the
 // order tiles finish in. A finalize kernel turns (sum n ln n, occupied bins)
 // into S2D and MI exactly as the histogram kernel's epilogue does.
+#include <limits.h>
 #include <math.h>
 #include <stdint.h>
 
@@ -245,6 +246,8 @@ struct OhSys {
     unsigned int *acc_occ;
     uint32_t *drain;  // INT32 totals of trajectories longer than a chunk: [slot][512 cols][128 rows]
     int F, R, D, drain_slots;
+    uint32_t *bits;   // one-bit masks (pg_onehot_bits.cuh): [K-block][row][8 words]
+    int nb, na, b2[3];  // DOFs of the first two types, 2D bins of each
 };
 
 // Per (row, chunk) item of the one-hot build, fixed for the whole K loop.
@@ -673,6 +676,8 @@ onehot_kernel(const OhSys *__restrict__ systems, const TcTile *__restrict__ tile
     }
 }
 
+#include "pg_onehot_bits.cuh"
+
 // S2D and MI of every pair from the accumulators (the histogram kernel's
 // epilogue formula): S = ln N + A_i + A_j - (1/N) sum n ln n + (occ-1)/(2N).
 // One system per blockIdx.z.
@@ -746,9 +751,15 @@ static int device_nsmid() {
 struct OnehotPlan {
     int64_t R = 0, n_tiles = 0;
     size_t off_rowstart = 0, off_rowinfo = 0, off_tiles = 0, off_fix = 0, off_snl = 0, off_occ = 0, off_sys = 0,
-           off_fin = 0, off_drain = 0, total = 0;
+           off_fin = 0, off_drain = 0, off_bits = 0, total = 0;
     int drain_slots = 0;
 };
+
+// The kernel of a launch: the masks' (pg_onehot_bits.cuh), or the FP8 build in
+// CTA pairs or single CTAs.
+enum Kind { OH_SINGLE, OH_PAIR, OH_BITS };
+static int64_t tile_rows(Kind k) { return k == OH_SINGLE ? kM : 2 * kM; }
+static int64_t tile_cols(Kind k) { return k == OH_BITS ? kBitN : kN; }
 
 // INT32 totals: one slot per SM id when the trajectory is longer than a chunk
 static int drain_slots_for(int F) { return F > kChunkFrames ? device_nsmid() : 0; }
@@ -764,27 +775,48 @@ static std::vector<uint32_t> rowinfo_of(const SysGeom &g) {
     return ri;
 }
 
-// pair: tiles of 256 rows (a CTA pair each), else 128; tiles tagged `sys`
-static OnehotPlan plan(const SysGeom &g, std::vector<TcTile> *tiles, bool pair = false, int sys = 0) {
+static int64_t rows_of(const SysGeom &g) {
+    return (int64_t)g.nb * g.bins[3 + TB] + (int64_t)g.na * g.bins[3 + TA] + (int64_t)g.nd * g.bins[3 + TD];
+}
+static size_t bits_bytes(const SysGeom &g) { return (size_t)rows_of(g) * ((g.F + kBitKB - 1) / kBitKB) * 32; }
+
+// The masks where they are held in 16 GB and the counts in their accumulators
+// (PG_ONEHOT_PAIR names one of the FP8 kernels). 2,994 DOFs x 100k frames, FP8
+// and masks: 23.2 and 7.9 ms at 8 bins, 36.2 and 11.8 at 10, 79.5 and 26.3 at 15,
+// 137.6 and 44.7 at 20; x 10k frames 5.45 and 2.23, 11.9 and 4.92 at 10 and 15.
+bool onehot_bits(const std::vector<SysGeom> &gs) {
+    if (getenv("PG_ONEHOT_PAIR")) return false;
+    size_t sum = 0;
+    for (const SysGeom &g : gs) {
+        if (g.F > kBitMaxFrames) return false;
+        sum += bits_bytes(g);
+    }
+    return sum <= (size_t)16 << 30;
+}
+
+// tiles tagged `sys`
+static OnehotPlan plan(const SysGeom &g, std::vector<TcTile> *tiles, Kind kind, int sys = 0) {
     OnehotPlan p;
     std::vector<int64_t> rs((size_t)g.D + 1, 0);
     for (int d = 0; d < g.D; d++) rs[d + 1] = rs[d] + bins_of(g, d);
     p.R = rs[g.D];
-    const int64_t tm = pair ? 2 * kM : kM;
-    const int64_t mts = (p.R + tm - 1) / tm, nts = (p.R + kN - 1) / kN;
+    const int64_t tm = tile_rows(kind), tn = tile_cols(kind);
+    const int64_t mts = (p.R + tm - 1) / tm, nts = (p.R + tn - 1) / tn;
     auto dof_at = [&](int64_t row) {  // last d with rs[d] <= row
         return (int)(std::upper_bound(rs.begin(), rs.end(), row) - rs.begin()) - 1;
     };
     int64_t cnt = 0;
-    for (int64_t mt = 0; mt < mts; mt++) {
-        const int rdof0 = dof_at(mt * tm);
+    // in strips of `strip` row tiles: the tiles that run together read few rows
+    const int64_t strip = kind == OH_BITS ? 8 : 1;
+    for (int64_t m0 = 0; m0 < mts; m0 += strip)
         for (int64_t nt = 0; nt < nts; nt++) {
-            const int64_t cend = std::min(p.R, (nt + 1) * kN) - 1;
-            if (dof_at(cend) <= rdof0) continue;  // no pair g1 < g2 in this tile
-            if (tiles) tiles->push_back(TcTile{(int)mt, (int)nt, sys, 0});
-            cnt++;
+            const int cdof = dof_at(std::min(p.R, (nt + 1) * tn) - 1);
+            for (int64_t mt = m0; mt < std::min(mts, m0 + strip); mt++) {
+                if (cdof <= dof_at(mt * tm)) continue;  // no pair g1 < g2 in this tile
+                if (tiles) tiles->push_back(TcTile{(int)mt, (int)nt, sys, 0});
+                cnt++;
+            }
         }
-    }
     p.n_tiles = cnt;
     p.off_rowstart = 0;
     p.off_rowinfo = al256(p.off_rowstart + sizeof(int64_t) * (g.D + 1));
@@ -795,8 +827,9 @@ static OnehotPlan plan(const SysGeom &g, std::vector<TcTile> *tiles, bool pair =
     p.off_sys = al256(p.off_occ + sizeof(unsigned int) * (size_t)g.D * g.D);
     p.off_fin = al256(p.off_sys + sizeof(OhSys));
     p.off_drain = al256(p.off_fin + sizeof(OhFin));
-    p.drain_slots = drain_slots_for(g.F);
-    p.total = al256(p.off_drain + sizeof(uint32_t) * kDrainSlotWords * (size_t)p.drain_slots);
+    p.drain_slots = kind == OH_BITS ? 0 : drain_slots_for(g.F);
+    p.off_bits = al256(p.off_drain + sizeof(uint32_t) * kDrainSlotWords * (size_t)p.drain_slots);
+    p.total = al256(p.off_bits + (kind == OH_BITS ? bits_bytes(g) : 0));
     return p;
 }
 
@@ -807,31 +840,40 @@ bool pairs_onehot_supported(const SysGeom &g) {
     return g.F >= 1;  // longer than one chunk (2^20 frames): INT32 totals across chunks
 }
 
-size_t pairs_onehot_scratch_bytes(const SysGeom &g) { return plan(g, nullptr).total; }
-
-// CTA pairs (tcgen05.mma.cta_group::2) unless PG_ONEHOT_PAIR=0 (one CTA per
-// 128 x 512 tile). Measured at 2,994 DOFs x 100k frames, 10 bins: 38.2 ms
+// The FP8 kernel in CTA pairs (tcgen05.mma.cta_group::2) unless
+// PG_ONEHOT_PAIR=0 (one CTA per 128 x 512 tile). Measured at 2,994 DOFs x 100k frames, 10 bins: 38.2 ms
 // against 54.7 ms.
 static bool use_pairs() {
     const char *e = getenv("PG_ONEHOT_PAIR");
     return !(e && atoi(e) == 0);
 }
+static Kind kind_of(bool bits) { return bits ? OH_BITS : use_pairs() ? OH_PAIR : OH_SINGLE; }
+
+size_t pairs_onehot_scratch_bytes(const SysGeom &g, bool bits) { return plan(g, nullptr, kind_of(bits)).total; }
 
 // The pair kernel over a tile list (each tile names its system) and the
 // finalize kernel over n_fin systems (largest D max_D).
-// low: every 2D bin count of the launch's systems is at most 64.
-static cudaError_t launch_tiles(const OhSys *d_sys, const TcTile *d_tiles, int64_t n_tiles, bool pair, bool low,
-                                const OhFin *d_fin, int n_fin, int max_D, int *err, cudaStream_t st) {
+// low: every 2D bin count of the launch's systems is at most 64. max_F: the
+// most frames of one.
+static cudaError_t launch_tiles(const OhSys *d_sys, const TcTile *d_tiles, int64_t n_tiles, Kind kind, bool low,
+                                const OhFin *d_fin, int n_fin, int max_D, int max_F, int *err, cudaStream_t st) {
     cudaError_t e;
     if (n_tiles > 0) {
-        if (pair) {
-            const size_t smem = (size_t)OhCfg<true>::kSmemBytes;
-            auto kern = low ? onehot_kernel<true, true> : onehot_kernel<true, false>;
+        if (kind == OH_BITS) {
+            const dim3 bg((unsigned)(((max_F + kBitKB - 1) / kBitKB * 8 + 255) / 256), max_D, n_fin);
+            onehot_bits_kernel<<<bg, 256, 0, st>>>(d_sys);
+            if ((e = cudaGetLastError())) return e;
+        }
+        if (kind != OH_SINGLE) {
+            const size_t smem = kind == OH_BITS ? (size_t)kBitSmem : (size_t)OhCfg<true>::kSmemBytes;
+            auto kern = kind == OH_BITS ? onehot_bits_pairs_kernel
+                        : low           ? onehot_kernel<true, true>
+                                        : onehot_kernel<true, false>;
             if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
                 return e;
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)(2 * n_tiles));
-            cfg.blockDim = dim3(kThreads);
+            cfg.blockDim = dim3(kind == OH_BITS ? kBitThreads : kThreads);
             cfg.dynamicSmemBytes = smem;
             cfg.stream = st;
             cudaLaunchAttribute at[1];
@@ -859,11 +901,11 @@ static cudaError_t launch_tiles(const OhSys *d_sys, const TcTile *d_tiles, int64
 // and the run (zeroed accumulators, pair kernel, finalize), which can be
 // repeated on the same inputs.
 cudaError_t onehot_setup(const SysGeom &g, const uint8_t *bins, const DofArrays &dof, PairOut out, cudaStream_t st,
-                         void *scratch, size_t scratch_bytes, OnehotRun *run) {
+                         void *scratch, size_t scratch_bytes, bool bits, OnehotRun *run) {
     if (!pairs_onehot_supported(g)) return cudaErrorInvalidValue;
-    const bool pair = use_pairs();
+    const Kind kind = kind_of(bits);
     std::vector<TcTile> tiles;
-    const OnehotPlan p = plan(g, &tiles, pair);
+    const OnehotPlan p = plan(g, &tiles, kind);
     if (scratch_bytes < p.total) return cudaErrorInvalidValue;
     char *base = (char *)scratch;
     const std::vector<uint32_t> ri = rowinfo_of(g);
@@ -874,7 +916,8 @@ cudaError_t onehot_setup(const SysGeom &g, const uint8_t *bins, const DofArrays 
     unsigned int *d_occ = (unsigned int *)(base + p.off_occ);
     const double fix = nlogn_fix_scale(g.F);  // per-bin rounding error 2^-(s+1)
     const OhSys hs{bins, g.ldb, d_ri, d_fix, d_snl, d_occ,
-                   p.drain_slots ? (uint32_t *)(base + p.off_drain) : nullptr, g.F, (int)p.R, g.D, p.drain_slots};
+                   p.drain_slots ? (uint32_t *)(base + p.off_drain) : nullptr, g.F, (int)p.R, g.D, p.drain_slots,
+                   (uint32_t *)(base + p.off_bits), g.nb, g.na, {g.bins[3], g.bins[4], g.bins[5]}};
     const OhFin hf{g, dof, d_snl, d_occ, out, log((double)g.F), fix};
     cudaError_t e;
     if ((e = cudaMemcpyAsync(d_ri, ri.data(), ri.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st))) return e;
@@ -892,7 +935,8 @@ cudaError_t onehot_setup(const SysGeom &g, const uint8_t *bins, const DofArrays 
     run->off_snl = p.off_snl;
     run->acc_bytes = p.off_sys - p.off_snl;  // the accumulators up to the descriptors
     run->n_tiles = p.n_tiles;
-    run->pair = pair;
+    run->kind = kind;
+    run->F = g.F;
     run->low = bmax2d(g) <= 64;
     run->D = g.D;
     return cudaSuccess;
@@ -903,39 +947,39 @@ cudaError_t onehot_run(const OnehotRun &run, int *err, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(base + run.off_snl, 0, run.acc_bytes, st);
     if (e != cudaSuccess) return e;
     return launch_tiles((const OhSys *)(base + run.off_sys), (const TcTile *)(base + run.off_tiles), run.n_tiles,
-                        run.pair, run.low, (const OhFin *)(base + run.off_fin), 1, run.D, err, st);
+                        (Kind)run.kind, run.low, (const OhFin *)(base + run.off_fin), 1, run.D, run.F, err, st);
 }
 
 cudaError_t launch_pairs_onehot(const SysGeom &g, const uint8_t *bins, const DofArrays &dof,
                                 const double *, PairOut out, int *err, cudaStream_t st, void *scratch,
-                                size_t scratch_bytes, int *launches) {
+                                size_t scratch_bytes, bool bits, int *launches) {
     *launches = 0;
     OnehotRun run;
-    cudaError_t e = onehot_setup(g, bins, dof, out, st, scratch, scratch_bytes, &run);
+    cudaError_t e = onehot_setup(g, bins, dof, out, st, scratch, scratch_bytes, bits, &run);
     if (e != cudaSuccess) return e;
-    *launches = 3;  // n ln n table, pair kernel, finalize
+    *launches = bits ? 4 : 3;  // n ln n table, masks, pair kernel, finalize
     return onehot_run(run, err, st);
 }
 
 // ---- many systems in one launch (pg_entropy_batch)
 //
 // Workspace: OhSys[n] | OhFin[n] | tiles | per system: rowinfo, n ln n table
-// | the accumulators of all systems, contiguous (one memset per run).
+// | the accumulators of all systems, contiguous (one memset per run) | masks.
 struct OhBatchLayout {
-    std::vector<size_t> off_ri, off_fix, off_snl, off_occ;
+    std::vector<size_t> off_ri, off_fix, off_snl, off_occ, off_bits;
     size_t off_sys = 0, off_fin = 0, off_tiles = 0, acc_begin = 0, acc_end = 0, off_drain = 0, total = 0;
     std::vector<TcTile> tiles;
     int max_D = 1, drain_slots = 0;
 };
 
-static OhBatchLayout batch_layout(const std::vector<SysGeom> &gs, bool pair) {
+static OhBatchLayout batch_layout(const std::vector<SysGeom> &gs, Kind kind) {
     OhBatchLayout L;
     const int n = (int)gs.size();
     // tiles of the systems with the most frames (the longest tiles) first
     std::vector<int> order((size_t)n);
     for (int s = 0; s < n; s++) order[s] = s;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return gs[a].F > gs[b].F; });
-    for (int s : order) plan(gs[s], &L.tiles, pair, s);
+    for (int s : order) plan(gs[s], &L.tiles, kind, s);
     size_t off = 0;
     L.off_sys = off;
     off = al256(off + sizeof(OhSys) * n);
@@ -966,23 +1010,26 @@ static OhBatchLayout batch_layout(const std::vector<SysGeom> &gs, bool pair) {
     L.acc_end = off;
     int maxF = 0;
     for (const SysGeom &g : gs) maxF = std::max(maxF, g.F);
-    L.drain_slots = drain_slots_for(maxF);
+    L.drain_slots = kind == OH_BITS ? 0 : drain_slots_for(maxF);
     L.off_drain = al256(off);
-    L.total = al256(L.off_drain + sizeof(uint32_t) * kDrainSlotWords * (size_t)L.drain_slots);
+    off = al256(L.off_drain + sizeof(uint32_t) * kDrainSlotWords * (size_t)L.drain_slots);
+    L.off_bits.resize(n);
+    for (int s = 0; s < n; s++) {
+        L.off_bits[s] = off;
+        if (kind == OH_BITS) off = al256(off + bits_bytes(gs[s]));
+    }
+    L.total = off;
     return L;
 }
 
-size_t pairs_onehot_batch_bytes(const std::vector<SysGeom> &gs) { return batch_layout(gs, use_pairs()).total; }
-
-int64_t pairs_onehot_batch_tiles(const std::vector<SysGeom> &gs) {
-    return (int64_t)batch_layout(gs, use_pairs()).tiles.size();
+size_t pairs_onehot_batch_bytes(const std::vector<SysGeom> &gs, bool bits) {
+    return batch_layout(gs, kind_of(bits)).total;
 }
 
 cudaError_t prepare_pairs_onehot_batch(const std::vector<SysGeom> &gs, const std::vector<const uint8_t *> &bins,
                                        const std::vector<DofArrays> &dofs, const std::vector<PairOut> &outs,
-                                       void *ws, size_t ws_bytes, cudaStream_t st) {
-    const bool pair = use_pairs();
-    const OhBatchLayout L = batch_layout(gs, pair);
+                                       void *ws, size_t ws_bytes, bool bits, cudaStream_t st) {
+    const OhBatchLayout L = batch_layout(gs, kind_of(bits));
     if (ws_bytes < L.total) return cudaErrorInvalidValue;
     const int n = (int)gs.size();
     char *base = (char *)ws;
@@ -998,7 +1045,8 @@ cudaError_t prepare_pairs_onehot_batch(const std::vector<SysGeom> &gs, const std
         hs[s] = OhSys{bins[s], g.ldb, (const uint32_t *)(base + L.off_ri[s]), (const int64_t *)(base + L.off_fix[s]),
                       (unsigned long long *)(base + L.off_snl[s]), (unsigned int *)(base + L.off_occ[s]),
                       L.drain_slots ? (uint32_t *)(base + L.off_drain) : nullptr, g.F, (int)ri[s].size(), g.D,
-                      L.drain_slots};
+                      L.drain_slots, (uint32_t *)(base + L.off_bits[s]), g.nb, g.na,
+                      {g.bins[3], g.bins[4], g.bins[5]}};
         hf[s] = OhFin{g, dofs[s], hs[s].acc_snl, hs[s].acc_occ, outs[s], log((double)g.F), fix};
         if ((e = cudaMemcpyAsync(base + L.off_ri[s], ri[s].data(), ri[s].size() * sizeof(uint32_t),
                                  cudaMemcpyHostToDevice, st)))
@@ -1014,21 +1062,24 @@ cudaError_t prepare_pairs_onehot_batch(const std::vector<SysGeom> &gs, const std
     return cudaStreamSynchronize(st);  // the host vectors go out of scope
 }
 
-cudaError_t launch_pairs_onehot_batch(const std::vector<SysGeom> &gs, void *ws, int *err, cudaStream_t st,
+cudaError_t launch_pairs_onehot_batch(const std::vector<SysGeom> &gs, void *ws, bool bits, int *err, cudaStream_t st,
                                       int *launches) {
-    const bool pair = use_pairs();
-    const OhBatchLayout L = batch_layout(gs, pair);
+    const Kind kind = kind_of(bits);
+    const OhBatchLayout L = batch_layout(gs, kind);
     char *base = (char *)ws;
     cudaError_t e = cudaMemsetAsync(base + L.acc_begin, 0, L.acc_end - L.acc_begin, st);
     if (e != cudaSuccess) return e;
-    *launches = 2;
-    int bmax = 1;
-    for (const SysGeom &g : gs) bmax = std::max(bmax, bmax2d(g));
+    *launches = bits ? 3 : 2;
+    int bmax = 1, max_F = 1;
+    for (const SysGeom &g : gs) {
+        bmax = std::max(bmax, bmax2d(g));
+        max_F = std::max(max_F, g.F);
+    }
     return launch_tiles((const OhSys *)(base + L.off_sys), (const TcTile *)(base + L.off_tiles),
-                        (int64_t)L.tiles.size(), pair, bmax <= 64, (const OhFin *)(base + L.off_fin), (int)gs.size(),
-                        L.max_D, err, st);
+                        (int64_t)L.tiles.size(), kind, bmax <= 64, (const OhFin *)(base + L.off_fin), (int)gs.size(),
+                        L.max_D, max_F, err, st);
 }
 
-int64_t pairs_onehot_tiles(const SysGeom &g) { return plan(g, nullptr, use_pairs()).n_tiles; }
+int64_t pairs_onehot_tiles(const SysGeom &g, bool bits) { return plan(g, nullptr, kind_of(bits)).n_tiles; }
 
 }  // namespace pg
