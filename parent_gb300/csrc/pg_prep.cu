@@ -11,6 +11,15 @@
 // with explicit round-to-nearest intrinsics (no FMA contraction), and this
 // file is compiled with --fmad=false, so bin indices equal the reference's
 // int((x - min) / binsize) on x86-64 (which never fuses).
+//
+// What bounds it: instructions and their latency (80 a value, half of the issue
+// slots; the column of 0.4 to 4 MB is read from L2 after the first pass). What
+// helped, FP32 input, 2,994 DOFs x 100k and 894 x 1M frames, 1.67 and 3.97 ms
+// before, 1.13 and 2.63 now: a threshold on the value in place of the shift's
+// quotient, with the extrema of two regions instead of three; a bin's error
+// bound from the sum that is rounded instead of the operands (the FP64 fallback
+// for 1 value in 20,000 instead of 1,400); one histogram where the 1D and 2D bin
+// counts are the same; the fallbacks out of line.
 #include <math.h>
 
 #include "pg_internal.h"
@@ -36,6 +45,13 @@ __device__ __forceinline__ double shifted(double x, double modfit, double twopi)
 
 __device__ __forceinline__ int bin_index(double x, double mn, double bs) {
     return __double2int_rz(__ddiv_rn(__dsub_rn(x, mn), bs));
+}
+
+// The exact decisions behind the screens, out of line: inlined into every
+// unrolled value their divisions made the loops miss the instruction cache.
+__device__ __noinline__ int exact_modfit(double x, double bs) { return __double2int_rz(__ddiv_rn(x, bs)); }
+__device__ __noinline__ int exact_shift(double x, double modfit, double twopi) {
+    return shift_quot(__dadd_rn(x, modfit), twopi);
 }
 
 // ---- FP32 screening of the FP64 bin decisions (FP32 input only).
@@ -75,8 +91,13 @@ __device__ __forceinline__ F2 split2(double v) {
 struct Bins {
     double mn, bs1, bs2;
     F2 mn2;
+    F2 o[2];  // FP32 input: the shift of either side of the threshold, less the minimum
     float r1, r2, e1, e2;
+    double modfit, twopi;
 };
+__device__ __noinline__ int exact_bin(double x, bool dih, const Bins &b, double bs) {
+    return bin_index(dih ? shifted(x, b.modfit, b.twopi) : x, b.mn, bs);
+}
 struct Consts {
     double modfit_bs, pi;
     float rm, r2pi;  // FP32 reciprocals of modfit_bs and 2 pi
@@ -104,35 +125,6 @@ __device__ __forceinline__ double okey_double(unsigned long long k) {
     const unsigned long long b = (k >> 63) ? (k & 0x7fffffffffffffffull) : ~k;
     return __longlong_as_double((long long)b);
 }
-
-// The same images for the input type: FP32 values keep 32-bit keys (the
-// conversion to FP64 is exact and monotone, so the same values win; only the
-// winners are converted), FP64 values the keys above.
-template <typename T>
-struct OKey;
-template <>
-struct OKey<float> {
-    using K = unsigned int;
-    static __device__ __forceinline__ K key(float x) {
-        unsigned int b = __float_as_uint(x);
-        if (b == 0x80000000u) b = 0u;
-        return (b >> 31) ? ~b : (b | 0x80000000u);
-    }
-    static __device__ __forceinline__ bool nan(float x) { return (__float_as_uint(x) & 0x7fffffffu) > 0x7f800000u; }
-    static __device__ __forceinline__ double value(unsigned long long k) {
-        const unsigned int c = (unsigned int)k;
-        return (double)__uint_as_float((c >> 31) ? (c & 0x7fffffffu) : ~c);
-    }
-    static constexpr K kNone = 0xffffffffu;
-};
-template <>
-struct OKey<double> {
-    using K = unsigned long long;
-    static __device__ __forceinline__ K key(double x) { return okey_raw(x); }
-    static __device__ __forceinline__ bool nan(double x) { return is_nan_bits(x); }
-    static __device__ __forceinline__ double value(unsigned long long k) { return okey_double(k); }
-    static constexpr K kNone = ~0ull;
-};
 
 // A column is streamed in runs of V = 16 / sizeof(T) consecutive frames, one
 // 16-byte load each, with U runs per thread in flight: one CTA streams a
@@ -208,9 +200,10 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
                : (const void *)((const float *)col + (int64_t)local * ld);
     const T *colT = (const T *)col;
     constexpr bool kDbl = sizeof(T) == 8;
-    // relative error bound factor of an FP32 quotient: 3 roundings (2^-23)
-    // for FP32 input, 4 for FP64 input rounded to FP32; both under 1/4 of it
-    constexpr float kQRel = kDbl ? 0x1p-20f : 0x1p-21f;
+    // relative error bound factors of the FP32 quotients, with a factor of 4 in
+    // hand: four roundings in a bin's (2^-22), three or two (FP32 input) in the
+    // modfit histogram's
+    constexpr float kQRel = 0x1p-20f, kMRel = kDbl ? 0x1p-20f : 0x1p-21f;
     const int F = geo.F;
     const int B1 = geo.bins[type], B2 = geo.bins[3 + type];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -224,6 +217,7 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
     __shared__ double s_shift;
     __shared__ Bins s_bins;
     __shared__ F2 s_mf2;
+    __shared__ float s_thr;  // FP32 dihedrals: the smallest value whose shift quotient is 1
 
     double modfit = 0.0;
     if (type == TD) {
@@ -236,8 +230,8 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
         for_frames<kUnroll, kThreads>(colT, F, tid, [&](int, T xv) {
             const float x = (float)xv;
             const float q = __fmul_rn(x, rm);
-            int idx = screened_floor(q, __fmul_ru(q, kQRel));
-            if (idx < 0) idx = __double2int_rz(__ddiv_rn((double)xv, modfit_bs));
+            int idx = screened_floor(q, __fmul_ru(q, kMRel));
+            if (idx < 0) idx = exact_modfit((double)xv, modfit_bs);
             if (idx < 0 || idx >= kModfitBins) { bad++; idx = idx < 0 ? 0 : kModfitBins - 1; }
             atomicAdd(&hmod[warp * kModfitBins + idx], 1u);
         });
@@ -276,6 +270,15 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
             // modFit = 2 pi - (pos + 0.5) * binsize, PARENT.cpp:609
             s_shift = __dsub_rn(twopi, __dmul_rn(__dadd_rn((double)longestPos, 0.5), modfit_bs));
             s_mf2 = split2(s_shift);
+            if (!kDbl) {
+                // next to 2 pi - modFit, where a float is far wider than the
+                // rounding of the FP64 expression
+                float t = __double2float_rn(__dsub_rn(twopi, s_shift));
+                for (int k = 0; k < 4 && shift_quot(__dadd_rn((double)nextafterf(t, -1e30f), s_shift), twopi) >= 1; k++)
+                    t = nextafterf(t, -1e30f);
+                for (int k = 0; k < 4 && shift_quot(__dadd_rn((double)t, s_shift), twopi) < 1; k++) t = nextafterf(t, 1e30f);
+                s_thr = t;
+            }
         }
         __syncthreads();
         modfit = s_shift;
@@ -292,7 +295,7 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
     auto shift_q = [&](T xv, float &t32) -> int {
         t32 = __fadd_rn(__fadd_rn((float)xv, mf2.hi), mf2.lo);
         int q = screened_floor(__fmul_rn(t32, r2pi), kShiftEps);
-        if (q < 0) q = shift_quot(__dadd_rn((double)xv, modfit), twopi);
+        if (q < 0) q = exact_shift((double)xv, modfit, twopi);
         return q;
     };
 
@@ -301,11 +304,67 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
     // compare exactly as floats, FP64 values through their integer images),
     // then the shifted FP64 value of each candidate
     double lmax = -1.0e100, lmin = 1.0e100;
-    {
-        using Key = OKey<T>;
-        using K = typename Key::K;
+    if constexpr (!kDbl) {
+        // FP32: an accepted value's quotient is 0 or 1 (x < 2 pi, modFit < 2 pi
+        // - 0.03), 1 from the threshold on, so the regions are those below and
+        // from it; fminf and fmaxf pass over NaN
+        constexpr float kInf = __builtin_huge_valf();
+        const float thr = type == TD ? s_thr : kInf;
+        float x0 = kInf, x1 = -kInf, lo = -kInf, hi = kInf;  // extrema, largest below thr, smallest from it
+        if (type == TD)
+            for_frames<kUnroll, kThreads>(colT, F, tid, [&](int, T xv) {
+                const float x = (float)xv;
+                x0 = fminf(x0, x);
+                x1 = fmaxf(x1, x);
+                lo = fmaxf(lo, x < thr ? x : -kInf);
+                hi = fminf(hi, x >= thr ? x : kInf);
+            });
+        else
+            for_frames<kUnroll, kThreads>(colT, F, tid, [&](int, T xv) {
+                x0 = fminf(x0, (float)xv);
+                x1 = fmaxf(x1, (float)xv);
+            });
+        __shared__ float red[kWarps][4];
+        for (int o = 16; o > 0; o >>= 1) {
+            x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
+            x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
+            lo = fmaxf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fminf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        if (lane == 0) {
+            red[warp][0] = x0;
+            red[warp][1] = x1;
+            red[warp][2] = lo;
+            red[warp][3] = hi;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            for (int w = 1; w < kWarps; w++) {
+                x0 = fminf(x0, red[w][0]);
+                x1 = fmaxf(x1, red[w][1]);
+                lo = fmaxf(lo, red[w][2]);
+                hi = fminf(hi, red[w][3]);
+            }
+            auto region = [&](float a, float b) {  // its smallest and largest value
+                double va = (double)b, vb = (double)a;
+                if (type == TD) {
+                    va = shifted(va, modfit, twopi);
+                    vb = shifted(vb, modfit, twopi);
+                }
+                if (va > lmax) lmax = va;
+                if (vb < lmin) lmin = vb;
+            };
+            if (type != TD) {
+                if (x0 <= x1) region(x0, x1);
+            } else {
+                if (x0 < thr) region(x0, lo);
+                if (x1 >= thr) region(hi, x1);
+            }
+        }
+    } else {
+        using K = unsigned long long;
         K kmax[kRegions], kmin[kRegions];
-        for (int r = 0; r < kRegions; r++) { kmax[r] = 0; kmin[r] = Key::kNone; }
+        for (int r = 0; r < kRegions; r++) { kmax[r] = 0; kmin[r] = ~0ull; }
         for_frames<kUnroll, kThreads>(colT, F, tid, [&](int, T xv) {
             int r = 0;
             if (type == TD) {
@@ -313,8 +372,8 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
                 r = shift_q(xv, t32);
                 r = r < 0 ? 0 : (r >= kRegions ? kRegions - 1 : r);  // out of range: flagged above
             }
-            const bool nan = Key::nan(xv);
-            const K k = Key::key(xv);
+            const bool nan = is_nan_bits(xv);
+            const K k = okey_raw(xv);
 #pragma unroll
             for (int q = 0; q < kRegions; q++) {
                 if (q == r && !nan) {
@@ -336,13 +395,13 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
         __syncthreads();
         if (tid == 0) {
             for (int q = 0; q < kRegions; q++) {
-                unsigned long long a = 0ull, b = Key::kNone;
+                unsigned long long a = 0ull, b = ~0ull;
                 for (int w = 0; w < kWarps; w++) {
                     a = red_kmax[w][q] > a ? red_kmax[w][q] : a;
                     b = red_kmin[w][q] < b ? red_kmin[w][q] : b;
                 }
                 if (a < b) continue;  // empty region
-                double va = Key::value(a), vb = Key::value(b);
+                double va = okey_double(a), vb = okey_double(b);
                 if (type == TD) {
                     va = shifted(va, modfit, twopi);
                     vb = shifted(vb, modfit, twopi);
@@ -372,19 +431,25 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
         b.mn = tmpMin;
         b.bs1 = __ddiv_rn(__dsub_rn(tmpMax, tmpMin), (double)B1);
         b.bs2 = __ddiv_rn(__dsub_rn(tmpMax, tmpMin), (double)B2);
-        // d = fl64(x' - mn) (x' the shifted value for dihedrals) is formed in
-        // FP32 from split constants, |d32 - d| <= 2^-20 E with
-        // E = |mn| + |mx| (+ 2|modFit| + 8 pi for dihedrals), a bound >= 4x
-        // the accumulated rounding (including an FP64 input's rounding to
-        // FP32, <= 2^-24 E); q_k = d32 * fl32(1 / bs_k) then has
-        // |q_k - q*| <= 2^-20 E / bs_k + 2^-22 q_k.
+        // d = fl64(x' - mn) (x' the shifted value for dihedrals). FP32 input:
+        // d32 = (x + o_hi) + o_lo with o = modFit - 2 pi q - mn in two floats,
+        // |d32 - d| <= 2^-23 |d| + 2^-46 E, E = |mn| + |mx| (+ 2|modFit| + 8 pi
+        // for dihedrals): the first sum rounds a number of d's size, no operand's.
+        // Then q_k = d32 * fl32(1 / bs_k) has |q_k - q*| <= 2^-22 q_k + 2^-46 E /
+        // bs_k. FP64 input is rounded to FP32 first, |d32 - d| <= 2^-22 E from
+        // split constants. All bounds are used with a factor of 4.
+        b.modfit = modfit;
+        b.twopi = twopi;
         b.mn2 = split2(tmpMin);
+        b.o[0] = split2(__dsub_rn(modfit, tmpMin));
+        b.o[1] = split2(__dsub_rn(__dsub_rn(modfit, twopi), tmpMin));
         b.r1 = __double2float_rn(__drcp_rn(b.bs1));
         b.r2 = __double2float_rn(__drcp_rn(b.bs2));
         double E = fabs(tmpMin) + fabs(tmpMax);
         if (type == TD) E = E + 2.0 * fabs(modfit) + 4.0 * twopi;
-        b.e1 = __double2float_ru(E * 0x1p-20 / b.bs1);
-        b.e2 = __double2float_ru(E * 0x1p-20 / b.bs2);
+        E = E * (kDbl ? 0x1p-20 : 0x1p-44);
+        b.e1 = __double2float_ru(E / b.bs1);
+        b.e2 = __double2float_ru(E / b.bs2);
         s_bins = b;
         dof.mn[g] = tmpMin;
         dof.mx[g] = tmpMax;
@@ -395,20 +460,23 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
     __syncthreads();
 
     // ---- binning (PARENT.cpp:654-656 1D; :800-803 and the other 2D fills)
-    const double mn = s_bins.mn, bs1 = s_bins.bs1, bs2 = s_bins.bs2;
+    const bool same = B1 == B2;  // one histogram for both
     int bad = 0;
     {
-        const F2 mn2 = s_bins.mn2;
+        const F2 mn2 = s_bins.mn2, o0 = s_bins.o[0], o1 = s_bins.o[1];
+        const float thr = !kDbl && type == TD ? s_thr : __builtin_huge_valf();
         const float r1 = s_bins.r1, r2 = s_bins.r2, e1 = s_bins.e1, e2 = s_bins.e2;
         // both bin indices of one value, counted in the 1D histograms; the 2D
         // bin is returned for the pair kernels' bin matrices
         auto bin_of = [&](T xin) -> int {
             const float x = (float)xin;
             float d32;
-            int q = 0;
-            if (type == TD) {
+            if constexpr (!kDbl) {
+                const bool up = x >= thr;
+                d32 = __fadd_rn(__fadd_rn(x, up ? o1.hi : o0.hi), up ? o1.lo : o0.lo);
+            } else if (type == TD) {
                 float t32;
-                q = shift_q(xin, t32);
+                const int q = shift_q(xin, t32);
                 const float qf = q >= 0 ? small_int_float(q) : (float)q;
                 d32 = __fsub_rn(__fsub_rn(__fsub_rn(__fsub_rn(t32, __fmul_rn(qf, tp2.hi)), __fmul_rn(qf, tp2.lo)),
                                           mn2.hi),
@@ -416,18 +484,20 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
             } else {
                 d32 = __fsub_rn(__fsub_rn(x, mn2.hi), mn2.lo);
             }
-            const float q1 = __fmul_rn(d32, r1), q2 = __fmul_rn(d32, r2);
-            int i1 = screened_floor(q1, __fadd_ru(e1, __fmul_ru(fabsf(q1), kQRel)));
-            int i2 = screened_floor(q2, __fadd_ru(e2, __fmul_ru(fabsf(q2), kQRel)));
+            const float q2 = __fmul_rn(d32, r2);
+            int i2 = screened_floor(q2, __fmaf_ru(fabsf(q2), kQRel, e2)), i1 = i2;
+            if (!same) {
+                const float q1 = __fmul_rn(d32, r1);
+                i1 = screened_floor(q1, __fmaf_ru(fabsf(q1), kQRel, e1));
+            }
             if (i1 < 0 || i2 < 0) {
-                double xv = (double)xin;
-                if (type == TD) xv = shift_apply(__dadd_rn(xv, modfit), q, twopi);
-                if (i1 < 0) i1 = bin_index(xv, mn, bs1);
-                if (i2 < 0) i2 = bin_index(xv, mn, bs2);
+                if (i2 < 0) i2 = exact_bin((double)xin, type == TD, s_bins, s_bins.bs2);
+                if (same) i1 = i2;
+                else if (i1 < 0) i1 = exact_bin((double)xin, type == TD, s_bins, s_bins.bs1);
             }
             if (i1 < 0 || i1 >= B1) { bad++; i1 = i1 < 0 ? 0 : B1 - 1; }
             if (i2 < 0 || i2 >= B2) { bad++; i2 = i2 < 0 ? 0 : B2 - 1; }
-            atomicAdd(&h1[w1 * B1 + i1], 1u);
+            if (!same) atomicAdd(&h1[w1 * B1 + i1], 1u);
             atomicAdd(&h2[warp * B2 + i2], 1u);
             return i2;
         };
@@ -449,13 +519,14 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
     }
     if (bad) atomicAdd(&err[ERR_BIN_RANGE], bad);
     __syncthreads();
-    for (int k = tid; k < B1 + B2; k += kThreads) {
+    for (int k = same ? B1 + tid : tid; k < B1 + B2; k += kThreads) {
         unsigned int *h = k < B1 ? h1 : h2;
         const int kk = k < B1 ? k : k - B1, stride = k < B1 ? B1 : B2;
         const int copies = k < B1 ? h1_copies : kWarps;
         unsigned int s = 0;
         for (int w = 0; w < copies; w++) s += h[w * stride + kk];
         h[kk] = s;
+        if (same) h1[kk] = s;
         if (k >= B1) dof.h2[(int64_t)g * kSegLd + kk] = (int)s;
     }
     __syncthreads();
@@ -465,6 +536,7 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
     // sines (each FP64 warp instruction costs the same with 1 or 32 lanes
     // active, and the FP64 pipe is a small fraction of this part's rate)
     if (warp == 0) {
+        const double mn = s_bins.mn, bs1 = s_bins.bs1, bs2 = s_bins.bs2;
         __shared__ double s_x[kTail], s_t[kTail];
         __shared__ unsigned char s_f[kTail];
         const int N = F;
