@@ -572,6 +572,7 @@ static int run_sorted(pg_ctx *ctx, const SysGeom &g, const DofArrays &dof, const
     d.list_ld = ld;
     d.pad = sorted_pad(g.D);
     a.joint = sorted_joint({g});
+    a.halves = !a.joint && sorted_halves(g);
     d.parts = sorted_parts(g, sorted_units(g.D), a.joint != 0);
     a.counter = (int *)ctx->sscr.p;
     a.ovf = (uint32_t *)((char *)ctx->sscr.p + 256);

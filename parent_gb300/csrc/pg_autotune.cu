@@ -328,7 +328,9 @@ static double tiled_seconds(const SysGeom &g) {
     return p * (9.96e-13 * F + 2.15e-8 + 3.9e-13 * b2);
 }
 static double sorted_seconds(const SysGeom &g, bool joint) {
-    const double u = (double)sorted_units(g.D), F = g.F, b = bmax_of(g);
+    // half a block takes 0.64 of one's time
+    const double u = sorted_units(g.D) - (!joint && sorted_halves(g) ? 0.36 * sorted_half_units(g.D) : 0.0);
+    const double F = g.F, b = bmax_of(g);
     if (joint) return u * (128 * 9.8e-14 * F + 1.5e-8 + 2.35e-11 * b * b * b) + 1.2e-11 * g.D * F;
     return u * (128 * (b < 118 ? 1.31e-13 : 1.62e-13) * F + 1e-8 + 6.4e-11 * b * b) + 9e-12 * g.D * F;
 }
@@ -338,6 +340,14 @@ static double sum_sorted(const std::vector<SysGeom> &gs, bool joint) {
     for (const SysGeom &g : gs) s += sorted_seconds(g, joint);
     return s;
 }
+
+// Half blocks on the diagonal, from 256 frames per row bin (the kernel's code is
+// larger, which short lists notice: 894 DOFs x 50 bins -0.6 % at 12k frames, -2.7
+// at 20k; 2,025 DOFs x 6.5k +1.9 %; 894 x 30 bins +0.5 % at 8k, -2.7 at 10k) to
+// blocks that L2 still holds (750k frames; with half the bytes in flight the
+// rows come from DRAM too late: 294 DOFs x 500k -9 %, 894 x 700k -2.9, 894 x 1M
+// +0.9). Single systems only: a batch of 16 took the same time either way.
+bool sorted_halves(const SysGeom &g) { return g.F >= 256 * bmax_of(g) && g.F <= 750000; }
 
 // Joint counters (PG_SORTED_JOINT=0|1 forces the choice where they fit).
 bool sorted_joint(const std::vector<SysGeom> &gs) {

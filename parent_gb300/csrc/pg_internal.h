@@ -285,17 +285,19 @@ struct SortedArgs {
     const unsigned long long *nfix;
     double fix;
     uint32_t *ovf;         // sorted_ovf_bytes, zeroed; each launch leaves it zeroed
-    int joint;             // sorted_joint
+    int joint, halves;     // sorted_joint, sorted_halves
     int bmax, half, rows, teams;  // set by the launchers
 };
 bool sorted_joint_fits(int bmax);
 bool sorted_joint(const std::vector<SysGeom> &gs);  // pg_autotune.cu
+bool sorted_halves(const SysGeom &g);
 int64_t sorted_list_ld(const SysGeom &g);
 int sorted_blocks(int D);
 size_t sorted_mat_bytes(const SysGeom &g);
 int sorted_pad(int D);
 size_t sorted_ovf_bytes(const SysGeom &g);
 int64_t sorted_units(int D);
+int64_t sorted_half_units(int D);
 int sorted_parts(const SysGeom &g, int64_t units, bool joint);
 void sorted_items(int s, int D, int row0, int row1, int parts, std::vector<SortedItem> &out);
 cudaError_t launch_sorted_transpose(const SortedArgs &a, int bmax, int max_F, const int2 *map, int n_blocks,

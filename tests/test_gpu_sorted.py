@@ -101,3 +101,26 @@ def test_sorted_batch_equals_single_calls(eng, monkeypatch, bins):
         bodies, trees = eng.entropy_batch(trajs, bins, "hist")
         for (flat, edges), body, (e, _) in zip(single, bodies, trees):
             assert np.array_equal(flat, body.flat()) and np.array_equal(edges, e)
+
+
+# half blocks on the diagonal: the first block wholly past its middle (pad of 64
+# columns and more), one short of it, a single block; segments around the pieces
+HALVES = [(66, 2000, (5, 7, 6), 0), (65, 4099, (16, 15, 14), 1), (67, 3001, (9, 8, 9), 0), (44, 13003, (50, 50, 50), 0),
+          (88, 5200, (20, 3, 1), 1), (47, 66000, (36, 50, 44), 0), (4, 999, (3, 3, 3), 0)]
+
+
+@pytest.mark.parametrize("atoms,frames,b2,prec", HALVES)
+def test_half_blocks_equal_tiled_and_oracle(eng, monkeypatch, atoms, frames, b2, prec):
+    monkeypatch.setenv("PG_SORTED_JOINT", "0")
+    test_sorted_equals_tiled_and_oracle(eng, monkeypatch, atoms, frames, b2, prec)
+
+
+@pytest.mark.parametrize("frames", [64512, 140000])
+def test_half_blocks_counts_above_16_bits(eng, monkeypatch, frames):
+    """66 DOFs (no row needs a lower column's counter), one value in most frames."""
+    monkeypatch.setenv("PG_SORTED_JOINT", "0")
+    t = pg.synth_host(24, frames, double_prec=0, seed=5)
+    for k, c in enumerate((t.bonds, t.angles, t.dihedrals)):
+        c[:, : frames - 7 - k] = c[:, :1]
+    (a, ea, _), (b, eb, _) = _both(eng, monkeypatch, t, (30,) * 6)
+    assert np.array_equal(a, b) and np.array_equal(ea, eb)
