@@ -24,6 +24,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <algorithm>
+
 #include "pg_internal.h"
 #include "pg_okey.cuh"
 
@@ -35,8 +37,9 @@ constexpr int kTie = 1 << 30;      // in bu: the row has its best value twice
 constexpr int kMergeThreads = 1024;
 constexpr int kScanWarps = 8;      // rows per CTA of a scan
 constexpr int kRankSplit = 8;      // CTAs sharing an edge's comparisons
+constexpr int kRoundMaxD = 4800;   // a wave of CTAs, the unions' arrays within the shared memory of one
 
-enum { CTL_FLAG = 0, CTL_NCOMP = 1, CTL_EDGES = 2 };
+enum { CTL_FLAG = 0, CTL_NCOMP = 1, CTL_EDGES = 2, CTL_ARRIVED = 3 };
 
 // One system's working arrays, after the 256 bytes of ctl (and before the
 // Prim kernels' own scratch).
@@ -71,8 +74,44 @@ __device__ __forceinline__ Tree tree_of(const MistDesc &d) {
     return t;
 }
 
+// What other threads wrote or write by atomics: of global memory (G) past L1
+template <bool G = true, typename T>
+__device__ __forceinline__ T fresh(const T *p) {
+    return G ? __ldcg(p) : *(const volatile T *)p;
+}
+template <bool G, typename T>
+__device__ __forceinline__ void put(T *p, T v) {
+    if (G) __stcg(p, v);
+    else *(volatile T *)p = v;
+}
+
+// t with the arrays of a round's unions, or all of them, at `at` in shared memory
+constexpr size_t kUnionBytes = 2 * sizeof(unsigned long long) + 4 * sizeof(int);  // per vertex
+constexpr size_t kTreeBytes = 4 * sizeof(unsigned long long) + 8 * sizeof(int);
+__device__ __forceinline__ Tree unions_at(Tree t, void *at) {
+    t.bkey = (unsigned long long *)at;
+    t.ckey = t.bkey + t.D;
+    t.bu = (int *)(t.ckey + t.D);
+    t.comp = t.bu + t.D;
+    t.win = t.comp + t.D;
+    t.parent = t.win + t.D;
+    return t;
+}
+__device__ __forceinline__ Tree tree_at(Tree t, void *at, int *ctl) {
+    t = unions_at(t, at);
+    t.ctl = ctl;
+    t.ek = (unsigned long long *)((char *)at + kUnionBytes * t.D);
+    t.ks = t.ek + t.D;
+    t.ea = (int *)(t.ks + t.D);
+    t.eb = t.ea + t.D;
+    t.rank = t.eb + t.D;
+    t.seq = t.rank + t.D;
+    return t;
+}
+
+template <bool G = true>
 __device__ __forceinline__ bool finished(const Tree &t) {
-    return __ldcg(t.ctl + CTL_FLAG) != 0 || __ldcg(t.ctl + CTL_NCOMP) <= 1;
+    return fresh<G>(t.ctl + CTL_FLAG) != 0 || fresh<G>(t.ctl + CTL_NCOMP) <= 1;
 }
 
 // Row v's best neighbour outside its component, by one warp; a neighbour found
@@ -129,20 +168,21 @@ __device__ __forceinline__ void scan_row(const Tree &t, int v, bool first, int l
 
 // One round's unions, by one CTA: every component's best row, its edge, the
 // new components.
+template <bool G>
 __device__ __forceinline__ void merge_round(const Tree &t) {
     const int tid = threadIdx.x, nthr = blockDim.x, D = t.D;
     __shared__ int s_bad, s_more, s_roots;
     if (tid == 0) s_bad = 0;
     for (int v = tid; v < D; v += nthr) {
-        __stcg(t.ckey + v, 0ull);
-        __stcg(t.win + v, -1);
+        put<G>(t.ckey + v, 0ull);
+        put<G>(t.win + v, -1);
     }
     __syncthreads();
     for (int v = tid; v < D; v += nthr) atomicMax(t.ckey + t.comp[v], t.bkey[v]);
     __syncthreads();
     for (int v = tid; v < D; v += nthr) {
         const int c = t.comp[v];
-        const unsigned long long k = __ldcg(t.ckey + c);
+        const unsigned long long k = fresh<G>(t.ckey + c);
         if (k == 0ull) s_bad = 1;  // nothing comparable leaves the component
         else if (t.bkey[v] == k && (atomicCAS(t.win + c, -1, v) != -1 || (t.bu[v] & kTie))) s_bad = 1;
     }
@@ -153,7 +193,7 @@ __device__ __forceinline__ void merge_round(const Tree &t) {
     }
     for (int c = tid; c < D; c += nthr) {
         if (t.comp[c] != c) continue;  // roots carry their component's number
-        const int v = __ldcg(t.win + c), u = t.bu[v], c2 = t.comp[u], w = __ldcg(t.win + c2);
+        const int v = fresh<G>(t.win + c), u = t.bu[v], c2 = t.comp[u], w = fresh<G>(t.win + c2);
         const bool mutual = w == u && t.bu[u] == v;  // the other component took the same edge
         if (!mutual || c < c2) {
             const int e = atomicAdd(t.ctl + CTL_EDGES, 1);
@@ -269,6 +309,7 @@ __device__ __forceinline__ void cta_scan(int *a, int n, int *s_scan) {
 //              1 + sum of the subtree sizes of a's heavier siblings.
 // Rooting is an Euler tour ranked by pointer doubling; the walks up the two
 // trees are short in trees of data and at most D steps.
+template <bool G>
 __device__ __forceinline__ void order_tree(const Tree &t, double *edge_mi, int *edge_from, int *edge_to) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_scan[33];
@@ -281,7 +322,7 @@ __device__ __forceinline__ void order_tree(const Tree &t, double *edge_mi, int *
     for (int k = tid; k < D + 1; k += nthr) start[k] = 0;
     __syncthreads();
     for (int e = tid; e < E; e += nthr) {
-        t.ks[__ldcg(t.rank + e)] = t.ek[e];
+        t.ks[fresh<G>(t.rank + e)] = t.ek[e];
         atomicAdd(&start[t.ea[e]], 1);
         atomicAdd(&start[t.eb[e]], 1);
     }
@@ -326,7 +367,7 @@ __device__ __forceinline__ void order_tree(const Tree &t, double *edge_mi, int *
         const int a = t.ea[e], b = t.eb[e];
         const bool down = (arc[sa[e]] >> 16) > (arc[sb[e]] >> 16);  // a -> b comes first
         // start is not read any more by anyone past the barrier above
-        up[down ? b : a] = (uint32_t)(down ? a : b) | (uint32_t)__ldcg(t.rank + e) << 16;
+        up[down ? b : a] = (uint32_t)(down ? a : b) | (uint32_t)fresh<G>(t.rank + e) << 16;
     }
     __syncthreads();
     int *size = (int *)arc;                          // subtree sizes, then the sums' terms, D
@@ -401,6 +442,7 @@ __device__ __forceinline__ void init_tree(const Tree &t, int i0, int stride) {
         t.ctl[CTL_FLAG] = 0;
         t.ctl[CTL_NCOMP] = t.D;
         t.ctl[CTL_EDGES] = 0;
+        t.ctl[CTL_ARRIVED] = 0;
     }
 }
 
@@ -421,13 +463,40 @@ __global__ void __launch_bounds__(kMergeThreads)
 tree_merge_kernel(const MistDesc *many, const __grid_constant__ MistDesc one) {
     const Tree t = tree_of(sys_of(many, one, blockIdx.x));
     if (finished(t)) return;
-    merge_round(t);
+    merge_round<true>(t);
+}
+
+// A round in one launch: 32 rows a CTA, and the last CTA to arrive makes the
+// unions, in shared memory.
+__global__ void __launch_bounds__(kMergeThreads)
+tree_round_kernel(const MistDesc *many, const __grid_constant__ MistDesc one, int first) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_last;
+    const Tree t = tree_of(sys_of(many, one, blockIdx.y));
+    if (finished(t)) return;  // the same for every CTA: set after the last one arrives
+    const int tid = threadIdx.x, v0 = blockIdx.x * (kMergeThreads / 32) + (tid >> 5);
+    if (v0 < t.D) scan_row(t, v0, first != 0, tid & 31);
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicInc((unsigned *)t.ctl + CTL_ARRIVED, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const Tree s = unions_at(t, smem);
+    for (int v = tid; v < t.D; v += kMergeThreads) {
+        s.bkey[v] = fresh(t.bkey + v);
+        s.bu[v] = fresh(t.bu + v);
+        s.comp[v] = t.comp[v];
+    }
+    __syncthreads();
+    merge_round<false>(s);
+    for (int v = tid; v < t.D; v += kMergeThreads) t.comp[v] = s.comp[v];
 }
 
 __global__ void __launch_bounds__(256) tree_rank_kernel(const MistDesc *many, const __grid_constant__ MistDesc one) {
     const Tree t = tree_of(sys_of(many, one, blockIdx.z));
     const int e = blockIdx.x * 256 + threadIdx.x, E = t.D - 1;
-    if (e >= E || __ldcg(t.ctl + CTL_NCOMP) != 1) return;
+    if (e >= E || fresh(t.ctl + CTL_NCOMP) != 1) return;
     const int per = (E + kRankSplit - 1) / kRankSplit, j0 = min(E, (int)blockIdx.y * per);
     rank_edge(t, e, j0, min(E, j0 + per));
 }
@@ -437,66 +506,75 @@ tree_order_kernel(const MistDesc *many, const __grid_constant__ MistDesc one) {
     const MistDesc d = sys_of(many, one, blockIdx.x);
     const Tree t = tree_of(d);
     // not one component, or not D - 1 edges: the Prim kernels take over
-    const bool whole = __ldcg(t.ctl + CTL_NCOMP) == 1 && __ldcg(t.ctl + CTL_EDGES) == t.D - 1;
-    if (!whole || __ldcg(t.ctl + CTL_FLAG)) {
+    const bool whole = fresh(t.ctl + CTL_NCOMP) == 1 && fresh(t.ctl + CTL_EDGES) == t.D - 1;
+    if (!whole || fresh(t.ctl + CTL_FLAG)) {
         if (threadIdx.x == 0) atomicExch(t.ctl + CTL_FLAG, 1);
         return;
     }
-    order_tree(t, d.edge_mi, d.edge_from, d.edge_to);
+    order_tree<true>(t, d.edge_mi, d.edge_from, d.edge_to);
 }
 
-// Everything in one CTA per system.
+// Everything in one CTA per system, in shared memory behind what the order needs.
 __global__ void __launch_bounds__(kMergeThreads)
 tree_small_kernel(const MistDesc *many, const __grid_constant__ MistDesc one) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int ctl[4];
     const MistDesc d = sys_of(many, one, blockIdx.x);
-    const Tree t = tree_of(d);
+    const Tree t = tree_at(tree_of(d), smem + (order_smem(d.D) + 15) / 16 * 16, ctl);
+    int *flag = (int *)d.scratch;
     const int tid = threadIdx.x;
     init_tree(t, tid, kMergeThreads);
     __syncthreads();
     for (int round = 0; round < 32; round++) {
         for (int v = tid >> 5; v < t.D; v += kMergeThreads / 32) scan_row(t, v, round == 0, tid & 31);
         __syncthreads();
-        merge_round(t);
+        merge_round<false>(t);
         __syncthreads();
-        if (finished(t)) break;  // the same for every thread: written before the barrier
+        if (finished<false>(t)) break;  // the same for every thread: written before the barrier
     }
     const int E = t.D - 1;
     __syncthreads();
-    if (__ldcg(t.ctl + CTL_FLAG) == 0 && __ldcg(t.ctl + CTL_NCOMP) == 1)
+    if (fresh<false>(t.ctl + CTL_FLAG) == 0 && fresh<false>(t.ctl + CTL_NCOMP) == 1)
         for (int e = tid; e < E; e += kMergeThreads) rank_edge(t, e, 0, E);
     __syncthreads();
-    const bool whole = __ldcg(t.ctl + CTL_NCOMP) == 1 && __ldcg(t.ctl + CTL_EDGES) == E;
-    if (!whole || __ldcg(t.ctl + CTL_FLAG)) {
-        if (tid == 0) atomicExch(t.ctl + CTL_FLAG, 1);
+    const bool whole = fresh<false>(t.ctl + CTL_NCOMP) == 1 && fresh<false>(t.ctl + CTL_EDGES) == E;
+    if (!whole || fresh<false>(t.ctl + CTL_FLAG)) {
+        if (tid == 0) *flag = 1;
         return;
     }
+    if (tid == 0) *flag = 0;
     __syncthreads();
-    order_tree(t, d.edge_mi, d.edge_from, d.edge_to);
+    order_tree<false>(t, d.edge_mi, d.edge_from, d.edge_to);
 }
 
-// One CTA to 256 vertices (144: 0.074 ms, 0.107 over the grid; 294: 0.138 and
-// 0.126).
-constexpr int kSmallD = 256;
+// One CTA to 224 vertices (189: 0.070 ms, 0.085 over the grid; 255: 0.090 and
+// 0.083).
+constexpr int kSmallD = 224;
 constexpr int kTreeMaxD = 16000;  // order_smem within a CTA's shared memory; arcs and distances in 16 bits
 
 }  // namespace
 
-// From 40 vertices on (18: 0.033 ms against Prim's 0.023, 66: 0.046 and 0.072).
+// From 16 vertices on (18: 0.019 ms against Prim's 0.021, 30: 0.023 and 0.032, 66:
+// 0.031 and 0.066).
 bool mist_tree_supported(int max_D) {
     if (getenv("PG_MIST_CLUSTER")) return false;  // a choice among the Prim kernels
-    return max_D >= 40 && max_D <= kTreeMaxD;
+    return max_D >= 16 && max_D <= kTreeMaxD;
 }
 
 size_t mist_tree_bytes(int D) { return 256 + (size_t)D * (4 * sizeof(unsigned long long) + 8 * sizeof(int)); }
 
-// All kernels of one tree, Prim's before: 294 DOFs 0.36 -> 0.13 ms, 603 0.92 ->
-// 0.15, 2,994 6.97 -> 0.33, 7,494 27.9 -> 0.86, 14,994 67.4 -> 2.1. At 7,494:
-// four scans 0.42 ms (450 MB of MI each, 3.6 TB/s), their unions 0.15, the
-// ranks 0.04, the order 0.15, rounds that find nothing left 0.08.
+// All kernels of one tree, Prim's before: 66 DOFs 0.066 -> 0.031 ms, 294 0.36 ->
+// 0.094, 603 0.92 -> 0.11, 2,994 6.97 -> 0.26, 7,494 27.9 -> 0.86, 14,994 67.4 ->
+// 2.1. Rounds of one launch with the unions in shared memory took the place of a
+// scan and a union on arrays in L2 to 4,800 DOFs (294 0.127 -> 0.094, 2,994 0.316
+// -> 0.261), as for the one-CTA form (66 0.043 -> 0.031). At 7,494: four scans
+// 0.42 ms (450 MB of MI each, 3.6 TB/s), their unions 0.15, the ranks 0.04, the
+// order 0.15, rounds that find nothing left 0.08.
 cudaError_t launch_mist_tree(const MistDesc *many, const MistDesc &one, int n_sys, int max_D, cudaStream_t st,
                              int *launches) {
-    const size_t smem = order_smem(max_D);
+    size_t smem = order_smem(max_D);
     if (max_D <= kSmallD) {
+        smem = (smem + 15) / 16 * 16 + kTreeBytes * max_D;
         cudaError_t e = cudaFuncSetAttribute(tree_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         tree_small_kernel<<<n_sys, kMergeThreads, smem, st>>>(many, one);
@@ -505,18 +583,28 @@ cudaError_t launch_mist_tree(const MistDesc *many, const MistDesc &one, int n_sy
     }
     cudaError_t e = cudaFuncSetAttribute(tree_order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
+    const bool fused = max_D <= kRoundMaxD;
+    const size_t unions = kUnionBytes * max_D;
+    if (fused) {
+        e = cudaFuncSetAttribute(tree_round_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)unions);
+        if (e != cudaSuccess) return e;
+    }
     const unsigned n = (unsigned)n_sys;
     tree_init_kernel<<<dim3((unsigned)((max_D + 255) / 256), n), 256, 0, st>>>(many, one);
     int rounds = 0;
     while ((1 << rounds) < max_D) rounds++;  // the components at least halve; the rounds left over return at once
     for (int r = 0; r < rounds; r++) {
+        if (fused) {
+            tree_round_kernel<<<dim3((unsigned)((max_D + 31) / 32), n), kMergeThreads, unions, st>>>(many, one, r == 0);
+            continue;
+        }
         tree_scan_kernel<<<dim3((unsigned)((max_D + kScanWarps - 1) / kScanWarps), n), kScanWarps * 32, 0, st>>>(many, one,
                                                                                                              r == 0);
         tree_merge_kernel<<<n, kMergeThreads, 0, st>>>(many, one);
     }
     tree_rank_kernel<<<dim3((unsigned)((max_D + 255) / 256), kRankSplit, n), 256, 0, st>>>(many, one);
     tree_order_kernel<<<n, kMergeThreads, smem, st>>>(many, one);
-    *launches += 3 + 2 * rounds;
+    *launches += 3 + (fused ? 1 : 2) * rounds;
     return cudaGetLastError();
 }
 

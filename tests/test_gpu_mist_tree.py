@@ -95,3 +95,15 @@ def test_ties_and_nan_are_prims(eng, monkeypatch, n_dih, kind):
     for f in e.dtype.names:
         assert np.array_equal(e[f], pe[f], equal_nan=f == "mi"), f
     assert np.array_equal(t, pt, equal_nan=True)
+
+
+# 15 and 18 DOFs, 222 and 225, 4,800 and 4,803: Prim's, one CTA, a launch per
+# round, scans and unions apart
+@pytest.mark.parametrize("n_dih", [4, 5, 73, 74, 1599, 1600])
+@pytest.mark.parametrize("shape", ["random", "zigzag chain"])
+def test_tree_kernels_meet_at_their_sizes(eng, monkeypatch, n_dih, shape):
+    body = _body(n_dih, _mi(shape, 3 * n_dih + 3, n_dih))
+    e, t = eng.mist(n_dih, body)
+    monkeypatch.setenv("PG_MIST_CLUSTER", "1")
+    pe, pt = eng.mist(n_dih, body)
+    assert np.array_equal(e, pe) and np.array_equal(t, pt)
