@@ -13,7 +13,8 @@
 // kernel (F = 4,096 and 16,384 or 32,768 frames, random bins, at least one full wave of
 // tiles), measured once per process, device and kernel variant. The form with
 // the smaller predicted time is picked; when probing is not possible the
-// measured crossover (one-hot up to 15 bins, from 4,096 frames) decides.
+// measured crossover (one-hot up to 15 bins, from 4,096 frames) decides. Sorted
+// lists have fitted times instead (below).
 #include <math.h>
 #include <stdint.h>
 #include <stdlib.h>
@@ -310,7 +311,8 @@ int hist_layout(const SysGeom &g) {
 // Sorted lists count whole blocks of 128 columns (2,994 DOFs: 1.04 slots a
 // pair, 603: 1.21, 294: 1.57) and read their counters once per row bin. Tiles
 // count pairs exactly, with 32-bit counters to 35 bins, 16-bit to 50, then 16
-// pairs a CTA, 4 from 58 bins and 1 above 100. Some of both, in ms:
+// pairs a CTA, 4 from 58 bins and 1 above 100. Some of both, in ms, the lists
+// without half blocks:
 //   2,994 DOFs x 100k: 10 bins 80.7 tiles, 68.8 lists, 51.5 joint; 20 bins 78.3,
 //     69.5, 60.1; 30 bins 76.7, 70.8, 77.6; 50 bins 90.5, 71.5; 64 bins 213, 75.0
 //   2,994 DOFs x 1k: 10 bins 4.12, 1.43, 2.02; 50 bins 8.09, 6.51
@@ -331,6 +333,11 @@ static double sorted_seconds(const SysGeom &g, bool joint) {
     // half a block takes 0.64 of one's time
     const double u = sorted_units(g.D) - (!joint && sorted_halves(g) ? 0.36 * sorted_half_units(g.D) : 0.0);
     const double F = g.F, b = bmax_of(g);
+    // above 20 bins a CTA holds one table of joint counters, and nothing counts
+    // while it is read out: 2,994 DOFs x 100k frames 59.0 ms at 20 bins, 67.3 at 21,
+    // 70.4 at 25, 76.6 at 30 (one column: 68.9 to 70.2); 894 x 500k 29.5, 29.9 at
+    // 22, 28.8 at 30 (34.6 to 33.9)
+    if (joint && b > 20) return u * (128 * 1.0e-13 * F + 4e-7 + 1.1e-11 * b * b * b) + 9e-12 * g.D * F;
     if (joint) return u * (128 * 9.8e-14 * F + 1.5e-8 + 2.35e-11 * b * b * b) + 1.2e-11 * g.D * F;
     return u * (128 * (b < 118 ? 1.31e-13 : 1.62e-13) * F + 1e-8 + 6.4e-11 * b * b) + 9e-12 * g.D * F;
 }
@@ -404,8 +411,9 @@ double predict_pair_seconds(const SysGeom &g, int form) {
 
 // The form for PG_FORM_AUTO: the one with the smaller predicted pair-kernel
 // time (PG_AUTOTUNE=0: the fixed crossover). Only geometries the one-hot form
-// supports and where it can win are probed: from 24 bins up one update costs
-// it 2 x 24^2 FP8 FLOPs, more than the histogram kernels' rate allows at the
+// supports and where it can win are probed: above 24 bins it loses (2,994 DOFs x
+// 100k frames: 65.0 ms against 68.8 at 24 bins, 71.9 and 70.3 at 25), as one
+// update costs it 2 x 24^2 FLOPs, all that the histogram kernels' rate allows at the
 // tensor cores' peak.
 int autotune_form(const SysGeom &g) {
     if (!pairs_onehot_supported(g)) return PG_FORM_HIST;
