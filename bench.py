@@ -76,7 +76,8 @@ def traffic_per_update(layout: str):
     """DRAM bytes per update of the pair kernel from the committed ncu capture
     (profiles/), or None: the capture is on a smaller case (2,994 DOFs x 100k
     frames) and is scaled by this launch's updates."""
-    name = {"stream32": "pairs_hist32s_kernel_precision_path_2994dof_100k_50bins.md",
+    name = {"sorted": "pairs_sorted_kernel_precision_path_2994dof_100k_50bins.md",
+            "stream32": "pairs_hist32s_kernel_precision_path_2994dof_100k_50bins.md",
             "ring32": "pairs_hist32_kernel_precision_path_2994dof_100k_30bins.md",
             "16": "pairs_hist_kernel_precision_path_2994dof_100k.md"}[layout]
     try:
@@ -88,8 +89,33 @@ def traffic_per_update(layout: str):
     return None, name
 
 
+def pair_layout(eng, n_dih: int, n_frames: int, bins: int) -> str:
+    """"sorted" where the library counts a system with sorted frame lists (its
+    prediction is then that of the forced choice), else the layout of its tiles."""
+    before = os.environ.get("PG_HIST_SORTED")
+    auto = eng.predict_pair_ms(n_dih, n_frames, (bins,) * 6, "hist")
+    os.environ["PG_HIST_SORTED"] = "1"
+    try:
+        chosen = eng.predict_pair_ms(n_dih, n_frames, (bins,) * 6, "hist") == auto
+    finally:
+        if before is None:
+            del os.environ["PG_HIST_SORTED"]
+        else:
+            os.environ["PG_HIST_SORTED"] = before
+    return "sorted" if chosen else hist_layout(bins)
+
+
+def onehot_rate(dofs: int, n_frames: int, bins: int) -> float:
+    """Dense tensor rate of the one-hot kernel the library takes, in bf16 rates:
+    packed FP4 where the one-bit masks fit in 16 GB, else FP8
+    (parent_gb300/csrc/pg_pairs_onehot.cu onehot_bits)."""
+    masks = dofs * bins * -(-n_frames // 256) * 32
+    fp4 = masks <= 16 << 30 and n_frames <= 1 << 22 and "PG_ONEHOT_PAIR" not in os.environ
+    return 4.0 if fp4 else 2.0
+
+
 def hist_layout(bins: int) -> str:
-    """The histogram layout the library picks (parent_gb300/csrc/pg_autotune.cu
+    """The layout of the tiled histogram kernels (parent_gb300/csrc/pg_autotune.cu
     hist_layout): the streamed 32-slot kernel up to 50 bins, else 16 slots;
     PG_HIST_SLOTS / PG_HIST_STREAM override it."""
     forced = os.environ.get("PG_HIST_SLOTS")
@@ -486,7 +512,9 @@ def run_batch(args):
             "config": {"workload": BATCH, "systems": len(systems), "dofs": [min(Ds), max(Ds)],
                        "frames": [min(Fs), max(Fs)], "updates_per_step": units, "input": "fp32",
                        "bins": args.bins, "form": batch_form,
-                       "hist_layout": hist_layout(args.bins) if batch_form == "hist" else None,
+                       "hist_layout": pair_layout(eng, max(a for a, _, _, _ in systems) - 3,
+                                                  max(f for _, f, _, _ in systems), args.bins)
+                       if batch_form == "hist" else None,
                        "parallelism": f"replicas x{world}" if world > 1 else "single gpu",
                        "l2": "inputs (%.1f GB) larger than L2; no flush" % (total_bytes / 1e9)},
             "sequential": {"ms_per_step": ms_seq, "value": units * world / (ms_seq / 1e3),
@@ -765,7 +793,8 @@ def run_gb300(args):
     if form == "hist":
         red_peak = eng.probe_smem_red_rate()
         achieved = units / pair_s
-        bpu, prof = traffic_per_update(hist_layout(args.bins))
+        layout = pair_layout(eng, n_dih, F, args.bins)
+        bpu, prof = traffic_per_update(layout)
         roofline = {"bound": "smem", "achieved": achieved / 1e9, "peak": red_peak / 1e9, "unit": "Gred/s",
                     "frac": achieved / red_peak, "traffic": bpu * units if bpu else None,
                     "note": "one shared-memory reduction per pair-frame update; peak = conflict-free "
@@ -774,10 +803,12 @@ def run_gb300(args):
                             "updates (bytes per launch)"}
     else:
         achieved = 2.0 * args.bins * args.bins * units / pair_s / 1e12
-        peak = 2.0 * float(peaks.get("bf16_tflops", 1900.0))
+        rate = onehot_rate(D, F, args.bins)
+        peak = rate * float(peaks.get("bf16_tflops", 1900.0))
         roofline = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                     "frac": achieved / peak, "traffic": None,
-                    "note": "2*B^2 one-hot FLOPs per update; peak = 2x measured cuBLAS bf16 (FP8 dense rate)"}
+                    "note": "2*B^2 one-hot FLOPs per update; peak = %.0fx measured cuBLAS bf16 (%s dense rate)"
+                            % (rate, "FP4" if rate > 2.0 else "FP8")}
     prep_s = statistics.mean(prep_ms) / 1e3
     hbm = float(peaks.get("hbm_gbs", 6800.0))
     prep_bytes = D * F * (es + 1)
@@ -798,7 +829,7 @@ def run_gb300(args):
             "vs_baseline": None, "dtype": "u32", "data": "synthetic",
             "config": {"workload": args.workload, "n_atoms": n_atoms, "dofs": D, "pairs": P, "frames": F,
                        "input": "fp64" if prec else "fp32", "bins": args.bins, "form": form,
-                       "hist_layout": hist_layout(args.bins) if form == "hist" else None,
+                       "hist_layout": layout if form == "hist" else None,
                        "parallelism": f"replicas x{world}" if world > 1 else "single gpu",
                        "l2": "inputs (%.1f GB) larger than L2; no flush" % (D * F * es / 1e9)},
             "kernel_ms": {"prep": statistics.mean(prep_ms), "pairs": statistics.mean(pair_ms),
@@ -821,16 +852,17 @@ def compare_forms(eng, view, n_dih: int, units: int, stream):
     50 and 10 bins, timed with CUDA events on the library's stream: the
     comparison the metric names (tensor-core one-hot against shared-memory
     histogram). The one-hot form's roofline is 2*B^2 FLOPs per update against
-    the dense FP8 rate, taken as 2x the measured sustained cuBLAS bf16 rate
-    (these are seconds-long kernels)."""
+    the dense rate of its operands, taken as 4x (FP4) or 2x (FP8) the measured
+    sustained cuBLAS bf16 rate (these are seconds-long kernels)."""
     import torch
     peaks = {}
     try:
         peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text())
     except (OSError, ValueError):
         pass
-    fp8 = 2.0 * float(peaks.get("bf16_tflops_sustained", 1700.0))
-    out = {"peak_fp8_tflops": fp8, "peak_note": "2x measured sustained cuBLAS bf16 (MEASURED_PEAKS.json)"}
+    bf16 = float(peaks.get("bf16_tflops_sustained", 1700.0))
+    out = {"peak_fp8_tflops": 2.0 * bf16, "peak_fp4_tflops": 4.0 * bf16,
+           "peak_note": "2x and 4x measured sustained cuBLAS bf16 (MEASURED_PEAKS.json)"}
     for b in (50, 10):
         row = {}
         for form in ("hist", "onehot"):
@@ -848,7 +880,8 @@ def compare_forms(eng, view, n_dih: int, units: int, stream):
             r = {"ms_per_step": ms, "pairs_ms": pair_ms, "value": units / (ms / 1e3), "form": eng.last_form()}
             if form == "onehot":
                 tf = 2.0 * b * b * units / (pair_ms / 1e3) / 1e12
-                r["roofline"] = {"bound": "tensor", "achieved": tf, "peak": fp8, "unit": "TFLOP/s", "frac": tf / fp8}
+                peak = bf16 * onehot_rate(3 * n_dih + 3, view.n_frames, b)
+                r["roofline"] = {"bound": "tensor", "achieved": tf, "peak": peak, "unit": "TFLOP/s", "frac": tf / peak}
             row[form] = r
         row["hist_over_onehot_time"] = row["hist"]["ms_per_step"] / row["onehot"]["ms_per_step"]
         out[str(b)] = row

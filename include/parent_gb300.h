@@ -53,8 +53,8 @@ typedef enum pg_status {
 /* Which pair-count kernel computes the 2D histograms. */
 typedef enum pg_form {
     PG_FORM_AUTO = 0,   /* autotuner picks per (bins, frames, DOFs) */
-    PG_FORM_HIST = 1,   /* shared-memory histogram kernel (TMA-staged bins, smem atomics) */
-    PG_FORM_ONEHOT = 2  /* tcgen05 one-hot GEMM kernel (FP8 0/1 operands, FP32 TMEM accumulate) */
+    PG_FORM_HIST = 1,   /* shared-memory histogram kernels (sorted frame lists or pair tiles) */
+    PG_FORM_ONEHOT = 2  /* tcgen05 one-hot GEMM kernels (FP4 or FP8 0/1 operands, FP32 TMEM accumulate) */
 } pg_form;
 
 typedef struct pg_ctx pg_ctx;
@@ -212,12 +212,13 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
 PG_API int pg_last_timings(const pg_ctx *ctx, double ms[5]);
 /* The autotuner's prediction (no reference counterpart) of the pair-kernel
  * milliseconds of a system of n_dihedrals / n_frames at these bins in a form
- * (PG_FORM_HIST with the histogram layout the library picks, PG_FORM_ONEHOT,
- * or PG_FORM_AUTO: the form the autotuner picks). The model is ceil(tiles /
- * concurrent tiles) x (t0 + t1 F) plus the form's per-call set-up, with t0,
- * t1 and the set-up measured on this GPU by short probe launches the first
- * time a kernel variant is needed (random bins, one full wave, F = 4,096 and
- * 32,768). PG_ERR_UNSUPPORTED if the form cannot run the geometry. */
+ * (PG_FORM_HIST with the histogram kernel the library picks, PG_FORM_ONEHOT,
+ * or PG_FORM_AUTO: the form the autotuner picks). Sorted lists are predicted
+ * from fitted times. The model of the others is ceil(tiles / concurrent tiles)
+ * x (t0 + t1 F) plus the form's per-call set-up, with t0, t1 and the set-up
+ * measured on this GPU by short probe launches the first time a kernel variant
+ * is needed (random bins, F = 4,096 and 16,384 or 32,768). PG_ERR_UNSUPPORTED
+ * if the form cannot run the geometry. */
 PG_API int pg_predict_pair_ms(pg_ctx *ctx, int n_dihedrals, int n_frames, const int bins[6], int form,
                               double *ms);
 /* Kernel launches issued by this context since creation. */
@@ -227,8 +228,8 @@ PG_API int pg_last_form(const pg_ctx *ctx);
 /* The context's CUDA stream (a cudaStream_t), for event timing by callers. */
 PG_API void *pg_stream(const pg_ctx *ctx);
 
-/* Debug/parity export: runs the same preprocessing and pair-histogram kernel
- * as pg_entropy for n_pairs explicit pairs (g1[k] < g2[k], global DOF
+/* Debug/parity export: runs the same preprocessing as pg_entropy and the tiled
+ * pair-histogram kernels for n_pairs explicit pairs (g1[k] < g2[k], global DOF
  * indices) and copies their 2D counts (row-major, B(g1) x B(g2), int64) to
  * counts + k*stride. The reference never exposes counts; this replaces
  * nothing and exists so counts can be compared bit-exactly. */

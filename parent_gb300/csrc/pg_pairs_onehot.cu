@@ -7,6 +7,10 @@
 // histogram of the pair, so the counts PARENT.cpp fills frame by frame
 // (e.g. :802-804) are entries of C.
 //
+// Two kernels: FP4 operands built from one-bit masks (pg_onehot_bits.cuh), the
+// default, and FP8 operands built from the bin bytes, for launches that the masks
+// do not hold (onehot_bits), as follows.
+//
 // A pair of CTAs (a cluster of 2, one per SM) computes one 256 x 512 tile of
 // C over all frames with tcgen05.mma.cta_group::2.kind::f8f6f4 (M=256, N=256,
 // K=32, two accumulators sharing the A tile): each CTA builds its 128 rows of

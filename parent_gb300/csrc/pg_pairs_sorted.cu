@@ -49,7 +49,7 @@
 // a quarter of one for the row bytes, a tenth for the frame numbers' shuffles.
 // 2,994 DOFs x 100k frames at 50 bins: pair phase 90.5 ms with the streamed
 // tiles (83 % busy at one and a half cycles and 6.7 instructions per 32
-// updates), 72.8 ms here, 0.6 ms of it the lists, 0.2 the transposition, 0.3
+// updates), 70.9 ms here, 0.6 ms of it the lists, 0.2 the transposition, 0.3
 // the finish.
 //
 // The counters stay below 128 KB: beyond that the lines that the loads bring
