@@ -15,7 +15,7 @@
 // What bounds it: instructions and their latency (80 a value, half of the issue
 // slots; the column of 0.4 to 4 MB is read from L2 after the first pass). What
 // helped, FP32 input, 2,994 DOFs x 100k and 894 x 1M frames, 1.67 and 3.97 ms
-// before, 1.13 and 2.63 now: a threshold on the value in place of the shift's
+// before, 1.13 and 2.63 with it: a threshold on the value in place of the shift's
 // quotient, with the extrema of two regions instead of three; a bin's error
 // bound from the sum that is rounded instead of the operands (the FP64 fallback
 // for 1 value in 20,000 instead of 1,400); one histogram where the 1D and 2D bin
@@ -243,41 +243,50 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
             hmod[k] = s;  // warp 0's row only read by thread k itself before this write
         }
         __syncthreads();
-        if (tid == 0) {
-            // longest circular stretch of empty bins, or the first minimum bin
-            // when none is empty (PARENT.cpp:573-608, including the run
-            // counter that starts at 2 because of the double increment)
-            const unsigned int *histo = hmod;
-            bool zeroExists = false;
-            for (int k = 0; k < kModfitBins; k++) zeroExists = zeroExists || (histo[k] == 0);
-            int longest = 0, longestPos = -1, cur = 0, curPos = 0;
-            if (zeroExists) {
-                for (int k = 0; k < 2 * kModfitBins; k++) {
-                    const int l = k % kModfitBins;
-                    if (cur == 0 && histo[l] == 0) { cur = 1; curPos = k; }
-                    if (cur > 0 && histo[l] == 0) cur += 1;
-                    if (cur > 0 && histo[l] != 0) {
-                        if (cur > longest) { longest = cur; longestPos = curPos; }
-                        cur = 0;
-                    }
-                }
-            } else {
-                longestPos = 0;
-                unsigned int mn = histo[0];
-                for (int k = 0; k < kModfitBins; k++)
-                    if (histo[k] < mn) { mn = histo[k]; longestPos = k; }
+        if (warp == 0) {
+            // longest circular stretch of empty bins (the first of equal ones), or
+            // the first minimum bin when none is empty (PARENT.cpp:573-608, whose
+            // run counter starts at 2 because of the double increment). A lane
+            // takes a stretch's start; the empty bins' bits, twice around
+            __shared__ uint32_t s_empty[8];
+            uint32_t lowest = 0xffffffffu;
+            for (int w = 0; w < 7; w++) {
+                const unsigned int n = hmod[(32 * w + lane) % kModfitBins];
+                const uint32_t e = __ballot_sync(0xffffffffu, n == 0u);
+                if (lane == 0) s_empty[w] = e;
+                lowest = min(lowest, n);
             }
-            // modFit = 2 pi - (pos + 0.5) * binsize, PARENT.cpp:609
-            s_shift = __dsub_rn(twopi, __dmul_rn(__dadd_rn((double)longestPos, 0.5), modfit_bs));
-            s_mf2 = split2(s_shift);
-            if (!kDbl) {
-                // next to 2 pi - modFit, where a float is far wider than the
-                // rounding of the FP64 expression
-                float t = __double2float_rn(__dsub_rn(twopi, s_shift));
-                for (int k = 0; k < 4 && shift_quot(__dadd_rn((double)nextafterf(t, -1e30f), s_shift), twopi) >= 1; k++)
-                    t = nextafterf(t, -1e30f);
-                for (int k = 0; k < 4 && shift_quot(__dadd_rn((double)t, s_shift), twopi) < 1; k++) t = nextafterf(t, 1e30f);
-                s_thr = t;
+            if (lane == 0) s_empty[7] = 0u;
+            __syncwarp();
+            lowest = __reduce_min_sync(0xffffffffu, lowest);
+            uint32_t best = 0u;  // length, then the earlier start
+            for (int k = lane; k < kModfitBins; k += 32) {
+                const int before = k > 0 ? k - 1 : kModfitBins - 1;
+                uint32_t n = lowest != 0u;  // none is empty: the minimum's first bin
+                if (lowest != 0u) n = hmod[k] == lowest;
+                else if ((s_empty[k >> 5] >> (k & 31) & 1u) && !(s_empty[before >> 5] >> (before & 31) & 1u))
+                    for (int w = k >> 5; w < 7; w++) {
+                        const uint32_t full = ~__funnelshift_r(s_empty[w], s_empty[w + 1], k & 31);
+                        const int run = full ? __ffs(full) - 1 : 32;
+                        n += run;
+                        if (run < 32) break;
+                    }
+                if (n) best = max(best, n << 8 | (uint32_t)(kModfitBins - 1 - k));
+            }
+            const int longestPos = kModfitBins - 1 - (int)(__reduce_max_sync(0xffffffffu, best) & 0xffu);
+            if (lane == 0) {
+                // modFit = 2 pi - (pos + 0.5) * binsize, PARENT.cpp:609
+                s_shift = __dsub_rn(twopi, __dmul_rn(__dadd_rn((double)longestPos, 0.5), modfit_bs));
+                s_mf2 = split2(s_shift);
+                if (!kDbl) {
+                    // next to 2 pi - modFit, where a float is far wider than the
+                    // rounding of the FP64 expression
+                    float t = __double2float_rn(__dsub_rn(twopi, s_shift));
+                    for (int k = 0; k < 4 && shift_quot(__dadd_rn((double)nextafterf(t, -1e30f), s_shift), twopi) >= 1; k++)
+                        t = nextafterf(t, -1e30f);
+                    for (int k = 0; k < 4 && shift_quot(__dadd_rn((double)t, s_shift), twopi) < 1; k++) t = nextafterf(t, 1e30f);
+                    s_thr = t;
+                }
             }
         }
         __syncthreads();
@@ -531,14 +540,17 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
     }
     __syncthreads();
 
-    // ---- per-DOF sums on warp 0: lane 0 runs the reference's sequential
-    // recurrences and sums, the 32 lanes take the per-bin logarithms and
-    // sines (each FP64 warp instruction costs the same with 1 or 32 lanes
-    // active, and the FP64 pipe is a small fraction of this part's rate)
-    if (warp == 0) {
+    // ---- per-DOF sums, the 1D ones on warp 0 and the 2D ones on warp 1: lane 0
+    // runs the reference's sequential recurrences and sums, the 32 lanes take the
+    // per-bin logarithms and sines (each FP64 warp instruction costs the same with
+    // 1 or 32 lanes active, and the FP64 pipe is a small fraction of this part's
+    // rate). Both chains at once, and the modfit stretches a lane each instead of
+    // one thread's 300 reads: 603 DOFs x 50k frames 0.163 -> 0.133 ms, 2,994 x 100k
+    // 1.13 -> 1.01, 294 x 20k FP64 0.094 -> 0.079.
+    if (warp < 2) {
         const double mn = s_bins.mn, bs1 = s_bins.bs1, bs2 = s_bins.bs2;
-        __shared__ double s_x[kTail], s_t[kTail];
-        __shared__ unsigned char s_f[kTail];
+        __shared__ double s_x2[2][kTail], s_t2[2][kTail];
+        double *s_x = s_x2[warp], *s_t = s_t2[warp];
         const int N = F;
         // lane 0: x_k = x_{k-1} + step for the bins [c0, c0 + n) (the
         // reference's repeated +=, carried across chunks in x)
@@ -550,50 +562,55 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
                 }
             __syncwarp();
         };
-        // lane 0: sum of the flagged terms in bin order, counting them
-        auto sum_terms = [&](double &sum, int &count, int n) {
+        // lane 0: sum of the terms in bin order; 0 (exact) for those left out
+        auto sum_terms = [&](double &sum, int n) {
             __syncwarp();
-            if (lane == 0)
-                for (int k = 0; k < n; k++)
-                    if (s_f[k]) {
-                        sum = sum + s_t[k];
-                        count++;
-                    }
+            if (lane == 0) {
+#pragma unroll 8
+                for (int k = 0; k < n; k++) sum = sum + s_t[k];
+            }
             __syncwarp();
         };
 
-        // 1D entropy in the reference's order (PARENT.cpp:658-670, 702-714, 746-756)
-        int occupbins = 0;
-        double plnpsum = 0.0, x1 = __dadd_rn(mn, bs1 / 2.0);
-        for (int c0 = 0; c0 < B1; c0 += kTail) {
-            const int n = min(kTail, B1 - c0);
-            if (type != TD) points(x1, bs1, n);
-            for (int k = lane; k < n; k += 32) {
-                const double h = (double)h1[c0 + k];
-                double probDens, t = 0.0;
-                if (type == TB) {
-                    const double blen = s_x[k];
-                    probDens = h / (((N * bs1) * blen) * blen);
-                    if (probDens > 0) t = ((blen * blen) * probDens) * log(probDens);
-                } else if (type == TA) {
-                    const double st = sin(s_x[k]);
-                    probDens = h / ((N * bs1) * st);
-                    if (probDens > 0) t = (st * probDens) * log(probDens);
-                } else {
-                    probDens = h / (N * bs1);
-                    if (probDens > 0) t = probDens * log(probDens);
+        if (warp == 0) {
+            // 1D entropy in the reference's order (PARENT.cpp:658-670, 702-714, 746-756)
+            int occupbins = 0;
+            double plnpsum = 0.0, x1 = __dadd_rn(mn, bs1 / 2.0);
+            for (int c0 = 0; c0 < B1; c0 += kTail) {
+                const int n = min(kTail, B1 - c0);
+                if (type != TD) points(x1, bs1, n);
+                for (int k = lane; k < n; k += 32) {
+                    const double h = (double)h1[c0 + k];
+                    double probDens, t = 0.0;
+                    if (type == TB) {
+                        const double blen = s_x[k];
+                        probDens = h / (((N * bs1) * blen) * blen);
+                        if (probDens > 0) t = ((blen * blen) * probDens) * log(probDens);
+                    } else if (type == TA) {
+                        const double st = sin(s_x[k]);
+                        probDens = h / ((N * bs1) * st);
+                        if (probDens > 0) t = (st * probDens) * log(probDens);
+                    } else {
+                        probDens = h / (N * bs1);
+                        if (probDens > 0) t = probDens * log(probDens);
+                    }
+                    s_t[k] = t;
+                    occupbins += probDens > 0;
                 }
-                s_t[k] = t;
-                s_f[k] = probDens > 0;
+                sum_terms(plnpsum, n);
             }
-            sum_terms(plnpsum, occupbins, n);
+            occupbins = __reduce_add_sync(0xffffffffu, occupbins);
+            if (lane == 0) {
+                plnpsum = -plnpsum * bs1;
+                dof.s1[g] = plnpsum + (occupbins - 1.0) / (2.0 * N);
+            }
+            return;
         }
 
         // A = ln(bs2) + (1/N) sum_k m(k) ln J(c_k), with c_k advanced by
         // repeated += binsize as the reference's 2D epilogues do
         // (e.g. PARENT.cpp:807-820); J = c^2 (bond), sin c (angle), 1 (dihedral).
         double acc = 0.0, x2 = __dadd_rn(mn, bs2 / 2.0);
-        int unused = 0;
         unsigned int m2 = 0;
         for (int c0 = 0; c0 < B2; c0 += kTail) {
             const int n = min(kTail, B2 - c0);
@@ -601,13 +618,15 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
             for (int k = lane; k < n; k += 32) {
                 const unsigned int h = h2[c0 + k];
                 m2 = h > m2 ? h : m2;
+                double t = 0.0;
                 if (type != TD && h) {
                     const double c = s_x[k];
-                    s_t[k] = (double)h * (type == TB ? log(c * c) : log(sin(c)));
+                    t = (double)h * (type == TB ? log(c * c) : log(sin(c)));
                 }
-                s_f[k] = type != TD && h != 0u;
+                s_t[k] = t;
             }
-            sum_terms(acc, unused, n);
+            if (type != TD) sum_terms(acc, n);
+            else __syncwarp();
         }
         // largest 2D-bin marginal count: no 2D bin of a pair with this DOF
         // can hold more frames
@@ -617,8 +636,6 @@ __device__ __forceinline__ void prep_body(const SysGeom &geo, const void *cb, co
         }
         if (lane == 0) {
             dof.m2[g] = (int)m2;
-            plnpsum = -plnpsum * bs1;
-            dof.s1[g] = plnpsum + (occupbins - 1.0) / (2.0 * N);
             dof.acon[g] = log(bs2) + acc / (double)N;
         }
     }

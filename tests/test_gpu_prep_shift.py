@@ -54,3 +54,32 @@ def test_shift_threshold(b1, b2):
     for k in oracle.BLOCKS:
         if ref[k].size:
             assert np.max(np.abs(body.blocks[k] - ref[k])) <= 1e-9, k
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_equal_stretches_and_minima(dtype):
+    """The first of equal empty stretches (inside the range, and one over its end),
+    the first of equal minima, and single bins empty or occupied."""
+    rng = np.random.default_rng(23)
+    n = 3000
+
+    def column(empty=(), low=()):
+        bins = np.array([b for b in range(100) if b not in empty])
+        each = np.where(np.isin(bins, low), 5, 20)
+        b = np.concatenate([np.repeat(bins, each), np.full(n - each.sum(), next(b for b in bins if b not in low))])
+        return ((b + 0.1 + 0.8 * rng.random(n)) * BS).astype(dtype)
+
+    cols = [column(low=(20, 70)), column(low=(0, 99)), column(empty=(10, 11, 12, 60, 61, 62)), column(empty=(98, 99, 0, 40, 41, 42)),
+            column(empty=(99, 0, 50, 51)), column(empty=(5,)), column(empty=range(3, 99)), column(empty=range(1, 100))]
+    nd = len(cols)
+    t = pg.Trajectory(rng.normal(1.4, 0.03, (nd + 2, n)).astype(dtype), rng.uniform(0.4, 2.7, (nd + 1, n)).astype(dtype),
+                      np.stack(cols))
+    with pg.Engine(0) as eng:
+        body = eng.entropy(t, (40,) * 3 + (50,) * 3, "hist")
+        shift = eng.dof_stats(3 * nd + 3)[2][2 * nd + 3:]
+    ref = oracle.parent(t.bonds, t.angles, t.dihedrals, (40,) * 3 + (50,) * 3)
+    starts = [20, 0, 10, 40, 50, 5, 3, 1]  # of 98-0 and 40-42, and of 99-0 and 50-51, the one that ends first
+    assert np.max(np.abs(shift - [2 * np.pi - (s + 0.5) * BS for s in starts])) <= 1e-12
+    for k in oracle.BLOCKS:
+        if ref[k].size:
+            assert np.max(np.abs(body.blocks[k] - ref[k])) <= 1e-9, k
