@@ -721,16 +721,20 @@ static int run_streamed(pg_ctx *ctx, const pg_bat_view *tv, pg_par_body *out) {
     char *cols = (char *)ctx->cols.p;
     const int lo[3] = {0, g.nb, g.nb + g.na}, cnt[3] = {g.nb, g.na, g.nd};
     const void *src[3] = {tv->bonds, tv->angles, tv->dihedrals};
+    const bool whole = tv->ld == F && K == 1;  // nothing to overlap: SM loads, the fastest route
+    if (whole && !pre) {
+        void *const dst[3] = {cols, cols + (size_t)lo[1] * F * es, cols + (size_t)lo[2] * F * es};
+        const size_t bytes[3] = {(size_t)cnt[0] * F * es, (size_t)cnt[1] * F * es, (size_t)cnt[2] * F * es};
+        int nl = 0;
+        CK(h2d_copy3(dst, src, bytes, cs, &nl));
+        ctx->launches += nl;
+    }
     for (int k = 0; k < K; k++) {
-        for (int t = 0; t < 3 && !pre; t++) {
+        for (int t = 0; t < 3 && !pre && !whole; t++) {
             const int a = std::max(G[k], lo[t]), b = std::min(G[k + 1], lo[t] + cnt[t]);
             if (a >= b) continue;
             const char *from = (const char *)src[t] + (size_t)(a - lo[t]) * tv->ld * es;
-            if (tv->ld == F && K == 1) {  // nothing to overlap: SM loads, the fastest route
-                bool pulled = false;
-                CK(h2d_copy(cols + (size_t)a * F * es, from, (size_t)(b - a) * F * es, cs, &pulled));
-                if (pulled) ctx->launches++;
-            } else if (tv->ld == F) {  // contiguous rows: one linear copy (2D copies ran at 20-80 GB/s)
+            if (tv->ld == F) {  // contiguous rows: one linear copy (2D copies ran at 20-80 GB/s)
                 CK(cudaMemcpyAsync(cols + (size_t)a * F * es, from, (size_t)(b - a) * F * es, cudaMemcpyHostToDevice,
                                    cs));
             } else
@@ -1982,18 +1986,19 @@ PG_API int pg_entropy_batch(pg_ctx *ctx, int n_sys, const pg_bat_view *trajs, co
         char *dst = arena + L.cols;
         const void *src[3] = {v.bonds, v.angles, v.dihedrals};
         const int cnt[3] = {L.g.nb, L.g.na, L.g.nd};
+        if ((size_t)v.ld == F) {
+            // pulled by SM loads where the GPU can read the host memory
+            // (about 3x the copy engine's rate here), else the copy engine
+            void *const to[3] = {dst, dst + (size_t)cnt[0] * F * es, dst + (size_t)(cnt[0] + cnt[1]) * F * es};
+            const size_t bytes[3] = {(size_t)cnt[0] * F * es, (size_t)cnt[1] * F * es, (size_t)cnt[2] * F * es};
+            int nl = 0;
+            CK(h2d_copy3(to, src, bytes, st, &nl));
+            ctx->launches += nl;
+            continue;
+        }
         for (int t = 0; t < 3; t++) {
             if (cnt[t] == 0) continue;
-            if ((size_t)v.ld == F) {
-                // pulled by SM loads where the GPU can read the host memory
-                // (about 3x the copy engine's rate here), else the copy engine
-                bool pulled = false;
-                CK(h2d_copy(dst, src[t], (size_t)cnt[t] * F * es, st, &pulled));
-                if (pulled) ctx->launches++;
-            } else {
-                CK(cudaMemcpy2DAsync(dst, F * es, src[t], (size_t)v.ld * es, F * es, cnt[t], cudaMemcpyHostToDevice,
-                                     st));
-            }
+            CK(cudaMemcpy2DAsync(dst, F * es, src[t], (size_t)v.ld * es, F * es, cnt[t], cudaMemcpyHostToDevice, st));
             dst += (size_t)cnt[t] * F * es;
         }
     }

@@ -19,6 +19,8 @@
 // they are loaded as two 32-bit words.
 #include <stdint.h>
 
+#include <algorithm>
+
 #include <type_traits>
 
 #include <cuda_runtime.h>
@@ -62,21 +64,28 @@ __global__ void __launch_bounds__(256) bat_transpose_kernel(const uint8_t *__res
     }
 }
 
-// dst[i] = src[i] for n 16-byte words; src is host memory the GPU can read
-// directly (pinned, or pageable where the platform maps it): the SMs pull it
-// over the host link, which on Grace-attached parts outruns a copy engine
-// (210 vs 120-210 GB/s measured, and unaffected by kernels running meanwhile)
-__global__ void __launch_bounds__(512) host_pull_kernel(const uint4 *__restrict__ src, uint4 *__restrict__ dst,
-                                                        size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        dst[i] = src[i];
+// dst[i] = src[i] for n 16-byte words of up to three blocks; src is host memory
+// the GPU can read directly (pinned, or pageable where the platform maps it): the
+// SMs pull it over the host link, which on Grace-attached parts outruns a copy
+// engine (210 vs 120-210 GB/s measured, and unaffected by kernels running
+// meanwhile). One launch for a trajectory's three blocks (0.35 MB each: 3 x 4.6 us
+// apart, 8.3 together, and two launches fewer).
+struct Pull {
+    const uint4 *src[3];
+    uint4 *dst[3];
+    size_t n[3];
+};
+__global__ void __launch_bounds__(512) host_pull_kernel(const __grid_constant__ Pull p) {
+    const size_t n01 = p.n[0] + p.n[1], n = n01 + p.n[2];
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        if (i < p.n[0]) p.dst[0][i] = p.src[0][i];
+        else if (i < n01) p.dst[1][i - p.n[0]] = p.src[1][i - p.n[0]];
+        else p.dst[2][i - n01] = p.src[2][i - n01];
+    }
 }
 
 }  // namespace
 
-// Copies `bytes` from host memory to the device with a pull kernel when the
-// GPU can read `src` directly and both addresses and the size are 16-byte
-// multiples; with a copy-engine copy otherwise. *pulled says which.
 bool host_readable(const void *src) {
     bool readable = false;
     cudaPointerAttributes at;
@@ -92,18 +101,45 @@ bool host_readable(const void *src) {
     return readable;
 }
 
-cudaError_t h2d_copy(void *dst, const void *src, size_t bytes, cudaStream_t st, bool *pulled) {
-    *pulled = false;
-    if (bytes == 0) return cudaSuccess;
-    const bool aligned = (((uintptr_t)dst | (uintptr_t)src | bytes) & 15) == 0;
-    const bool readable = aligned && host_readable(src);
-    if (!readable) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+// Copies up to three blocks (empty ones have no bytes) from host memory to the
+// device: those that the GPU can read directly, with both addresses and the size
+// 16-byte multiples, with one pull kernel, the others with copy-engine copies.
+cudaError_t h2d_copy3(void *const dst[3], const void *const src[3], const size_t bytes[3], cudaStream_t st,
+                      int *launches) {
+    Pull p{};
+    size_t total = 0;
+    for (int t = 0; t < 3; t++) {
+        if (bytes[t] == 0) continue;
+        const bool aligned = (((uintptr_t)dst[t] | (uintptr_t)src[t] | bytes[t]) & 15) == 0;
+        if (aligned && host_readable(src[t])) {
+            p.src[t] = (const uint4 *)src[t];
+            p.dst[t] = (uint4 *)dst[t];
+            p.n[t] = bytes[t] / 16;
+            total += p.n[t];
+        } else {
+            const cudaError_t e = cudaMemcpyAsync(dst[t], src[t], bytes[t], cudaMemcpyHostToDevice, st);
+            if (e != cudaSuccess) return e;
+        }
+    }
+    if (total == 0) return cudaSuccess;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    host_pull_kernel<<<4 * sms, 512, 0, st>>>((const uint4 *)src, (uint4 *)dst, bytes / 16);
-    *pulled = true;
+    const unsigned grid = (unsigned)std::min<size_t>((size_t)4 * sms, (total + 511) / 512);
+    host_pull_kernel<<<grid, 512, 0, st>>>(p);
+    ++*launches;
     return cudaGetLastError();
+}
+
+// One block; *pulled says which way.
+cudaError_t h2d_copy(void *dst, const void *src, size_t bytes, cudaStream_t st, bool *pulled) {
+    void *const d[3] = {dst, nullptr, nullptr};
+    const void *const s[3] = {src, nullptr, nullptr};
+    const size_t n[3] = {bytes, 0, 0};
+    int launches = 0;
+    const cudaError_t e = h2d_copy3(d, s, n, st, &launches);
+    *pulled = launches > 0;
+    return e;
 }
 
 // raw: nf records of rec bytes on the device; values start at byte off0 of a

@@ -321,6 +321,7 @@ cudaError_t launch_bat_phase(double *dtmp, int64_t ldt, int nf, int nd, const in
 // Host -> device copy by SM loads where the GPU can read the host memory
 // (pg_ingest.cu), else by the copy engine.
 cudaError_t h2d_copy(void *dst, const void *src, size_t bytes, cudaStream_t st, bool *pulled);
+cudaError_t h2d_copy3(void *const dst[3], const void *const src[3], const size_t bytes[3], cudaStream_t st, int *launches);
 // Host memory this GPU's kernels can read directly: pinned, or pageable where
 // the device has pageable memory access (a Grace-attached part).
 bool host_readable(const void *src);
